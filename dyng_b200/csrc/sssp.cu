@@ -292,7 +292,7 @@ __device__ __forceinline__ void offer_owner(const SsspParams& p, Ctx& X, int own
 
 // The push split in two stages, so that a lane issues the loads of several slots before it
 // commits any of them: prepare computes the offer and loads the target's current word; commit
-// does the atomicMin and the frontier bookkeeping (the same steps as visit<kPush>).
+// does the atomicMins and the frontier bookkeeping.
 struct Offer {
   int dst;
   u64 cand;
@@ -313,28 +313,47 @@ __device__ __forceinline__ void push_prepare(const SsspParams& p, Ctx& X, int u,
   r.cur = ld_cg(&p.packed[y]);
 }
 
-__device__ __forceinline__ void push_commit(const SsspParams& p, Ctx& X, const Offer& r) {
-  if (r.cand >= r.cur) return;  // also skips "no offer" (cand == INF)
-  const int dst = r.dst;
-  const u64 nd = X.pk.dist(r.cand);
-  const bool near = nd < X.threshold;
-  ++X.tries;
-  // The atomicMin, the claim (of the next near frontier, or of the far pile) and the row length
-  // are independent: issued together, they cost one round trip instead of three.  The claim is
-  // taken on the offer alone (the target's word read before was larger): when another lane's
-  // smaller word wins the atomicMin meanwhile, the vertex is still appended and is pushed once
-  // more with its current word -- redundant, never wrong.
-  const int len = near ? p.g.out_desc[dst].len : 0;
-  const u64 old = atomicMin(&p.packed[dst], r.cand);
-  const bool claimed = near ? claim(p.stamp, dst, X.gen) : atomicExch(&p.in_far[dst], 1) == 0;
-  if (r.cand < old) {
-    ++X.atomics;
-    touch(p, dst);
+// The commits of a lane's N offers together: every offer's atomicMin, claim (of the next near
+// frontier, or of the far pile) and target row length are issued before the result of any of them
+// is looked at, so a lane pays one round trip to L2 for all of them instead of one per offer.  The
+// claim is taken on the offer alone (the target's word read before was larger): when another
+// lane's smaller word wins the atomicMin meanwhile, the vertex is still appended and is pushed
+// once more with its current word -- redundant, never wrong.
+template <int N>
+__device__ __forceinline__ void push_commit(const SsspParams& p, Ctx& X, const Offer (&r)[N]) {
+  bool any = false;
+#pragma unroll
+  for (int q = 0; q < N; ++q) any |= r[q].cand < r[q].cur;
+  if (!any) return;
+  u64 old[N];
+  int mark[N], len[N];
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    old[q] = 0;
+    mark[q] = 0;
+    len[q] = 0;
+    if (r[q].cand >= r[q].cur) continue;  // also skips "no offer" (cand == INF)
+    const int dst = r[q].dst;
+    const bool near = X.pk.dist(r[q].cand) < X.threshold;
+    if (near) len[q] = p.g.out_desc[dst].len;
+    old[q] = atomicMin(&p.packed[dst], r[q].cand);
+    mark[q] = atomicExch(near ? &p.stamp[dst] : &p.in_far[dst], near ? X.gen : 1);
   }
-  if (!claimed) return;
-  ++X.appends;
-  if (near) list_append(X.next, dst, len, p.heavy_degree);
-  else staged_append(kStFar, X.far, X.far_cnt, dst);
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    if (r[q].cand >= r[q].cur) continue;
+    const int dst = r[q].dst;
+    const bool near = X.pk.dist(r[q].cand) < X.threshold;
+    ++X.tries;
+    if (r[q].cand < old[q]) {
+      ++X.atomics;
+      touch(p, dst);
+    }
+    if (near ? mark[q] == X.gen : mark[q] != 0) continue;  // already in the list
+    ++X.appends;
+    if (near) list_append(X.next, dst, len[q], p.heavy_degree);
+    else staged_append(kStFar, X.far, X.far_cnt, dst);
+  }
 }
 
 template <int MODE>
@@ -378,15 +397,12 @@ __device__ __forceinline__ void warp_slots(const SsspParams& p, Ctx& X, int owne
       const int e = grp << 2;
       const int4 c4 = __ldg(reinterpret_cast<const int4*>(col + e));
       const int4 w4 = __ldg(reinterpret_cast<const int4*>(wt + e));
-      Offer r0, r1, r2, r3;
-      push_prepare(p, X, owner, odu, e + 0 < e1 ? c4.x : -1, w4.x, r0);
-      push_prepare(p, X, owner, odu, e + 1 < e1 ? c4.y : -1, w4.y, r1);
-      push_prepare(p, X, owner, odu, e + 2 < e1 ? c4.z : -1, w4.z, r2);
-      push_prepare(p, X, owner, odu, e + 3 < e1 ? c4.w : -1, w4.w, r3);
-      push_commit(p, X, r0);
-      push_commit(p, X, r1);
-      push_commit(p, X, r2);
-      push_commit(p, X, r3);
+      Offer r[4];
+      push_prepare(p, X, owner, odu, e + 0 < e1 ? c4.x : -1, w4.x, r[0]);
+      push_prepare(p, X, owner, odu, e + 1 < e1 ? c4.y : -1, w4.y, r[1]);
+      push_prepare(p, X, owner, odu, e + 2 < e1 ? c4.z : -1, w4.z, r[2]);
+      push_prepare(p, X, owner, odu, e + 3 < e1 ? c4.w : -1, w4.w, r[3]);
+      push_commit<4>(p, X, r);
     }
     return;
   }
@@ -452,8 +468,7 @@ __device__ __forceinline__ void warp_rows(const SsspParams& p, Ctx& X, int owner
           r[q].dst = -1;
         }
       }
-      push_commit(p, X, r[0]);
-      push_commit(p, X, r[1]);
+      push_commit<2>(p, X, r);
     }
     return;
   }

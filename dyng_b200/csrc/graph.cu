@@ -1560,7 +1560,7 @@ void Workspace::reserve_vertices(long long n_cap, cudaStream_t s) {
     b->reserve(n, s);
     DYNGB200_CUDA(cudaMemsetAsync(b->ptr, 0, n * sizeof(int), s));
   }
-  for (DevBuf<int>* b : {&flag, &in_far}) {
+  for (DevBuf<int>* b : {&near_stamp, &in_far}) {
     b->release();
     b->reserve(n, s);
     DYNGB200_CUDA(cudaMemsetAsync(b->ptr, 0, n * sizeof(int), s));
@@ -1622,8 +1622,9 @@ void Workspace::reserve_batch(long long ops, int k, cudaStream_t s) {
 }
 
 int Workspace::next_generation(int count, cudaStream_t s) {
-  if (generation > INT32_MAX / 2) {
+  if (generation > kMaxGeneration / 2) {
     DYNGB200_CUDA(cudaMemsetAsync(stamp.ptr, 0, stamp.count * sizeof(int), s));
+    DYNGB200_CUDA(cudaMemsetAsync(near_stamp.ptr, 0, near_stamp.count * sizeof(int), s));
     DYNGB200_CUDA(cudaMemsetAsync(touch_stamp.ptr, 0, touch_stamp.count * sizeof(int), s));
     generation = 0;
   }

@@ -142,14 +142,16 @@ struct UpdateCtl {
   int walk_cnt[3];      // subtree-walk levels
   int walk_med_cnt[3];
   int cand_med_count;   // medium pull candidates
-  int far_count, far2_count;
+  int far_cnt[3];       // the far pile, its successor and a cleared one, by threshold raises
+  int generations_spent;  // the claims of the near-far loop started over in this call
+  u64 far_min[3];       // smallest distance a threshold raise left on the far pile
   u64 heavy_cnt[3];     // (slots << 40 | chunks) of the heavy near-frontier lists
   u64 walk_heavy[3];
   u64 pull_heavy;       // heavy pull candidates
   // push steps hand out medium rows and heavy chunks to warps through these cursors (per step,
   // triple-buffered like the list counters)
   int med_cursor[3];
-  int pad_cursor;
+  int local_rounds[3];  // the most rounds a block ran by itself inside a push step (same slots)
   unsigned long long heavy_cursor[3];
   int touched_count;
   int active[3];
@@ -173,9 +175,6 @@ struct UpdateCtl {
   long long feat_acc[4];
   float features[12];
   int sched_classes[3];  // the chosen class of each head (-1: no scheduler)
-  int loop_state[6];   // near-far state handed from block 0 back to the grid
-  long long loop_pushes;
-  u64 loop_threshold;
   // work counters (algorithmic traffic) and phase timestamps of the sssp kernel
   long long work[32];
   unsigned long long phase_ns[8];
@@ -192,13 +191,18 @@ struct UpdateCtl {
   alignas(128) unsigned bar_count;
   alignas(128) unsigned bar_gen;
   unsigned bar_err;  // the error word as the last arrival saw it (read after bar_gen moves)
-  // progress of a block that works alone (the small-frontier loop of block 0): the blocks waiting
+  // progress of a block that works alone (its own rounds of a near-far step): the blocks waiting
   // at a grid barrier meanwhile restart their time limit whenever it moves
   alignas(128) unsigned heartbeat;
 };
 
 // Persistent blocks the pointer-jumping survivor lists of the sssp kernel support.
 constexpr int kPjMaxBlocks = 1024;
+
+// Stamp generations: a claim of the near-far loop holds a generation and a block in one int.
+constexpr int kClaimBlockBits = 10;
+static_assert((1 << kClaimBlockBits) >= kPjMaxBlocks, "a claim names the block");
+constexpr int kMaxGeneration = (1 << (31 - kClaimBlockBits)) - 1;
 
 // Scratch memory of a context, sized on demand and reused (the reference's workspace pool).
 struct Workspace {
@@ -219,7 +223,7 @@ struct Workspace {
   // batch staging
   DevBuf<int32_t> b_ins_src, b_ins_dst, b_ins_w, b_del_src, b_del_dst;
   // sssp
-  DevBuf<int> stamp, touch_stamp, flag, in_far, ancestor;
+  DevBuf<int> stamp, touch_stamp, near_stamp, in_far, ancestor;
   DevBuf<int> pj_blk;  // per-block survivor counts of pointer jumping
   DevBuf<long long> batch_extrema;  // update_each: per-objective insertion weight range, max id
   DevBuf<int> candidates, frontier, near_a, near_b, far_a, far_b, heavy_a, heavy_b, pull_heavy,

@@ -56,7 +56,14 @@ __shared__ int g_nblk;  // blocks taking part in this launch (the schedule's gri
 __shared__ int g_bar_arrivals;  // arrivals a grid barrier waits for (g_nblk, plus test phantoms)
 __shared__ unsigned long long g_bar_limit;  // the barrier's time limit without progress (ns)
 
-__device__ __forceinline__ void staged_append(int id, int* list, int* count, int v) {
+__device__ __forceinline__ bool claim(int* stamp, int v, int generation) {
+  return atomicExch(&stamp[v], generation) != generation;
+}
+
+// `once` (with its generation): a claim that keeps an entry unique in the global list, for appends
+// that may name a vertex several times (nullptr: the caller's entries are unique already).
+__device__ __forceinline__ void staged_append(int id, int* list, int* count, int v,
+                                              int* once = nullptr, int once_gen = 0) {
   const unsigned mask = __activemask();
   const int lane = threadIdx.x & 31;
   const int leader = __ffs(mask) - 1;
@@ -70,7 +77,7 @@ __device__ __forceinline__ void staged_append(int id, int* list, int* count, int
   base = __shfl_sync(mask, base, leader);
   const int pos = base + rank;
   if (pos < kStageCap) g_stage.data[id][pos] = v;
-  else list[append_slot(count)] = v;
+  else if (!once || claim(once, v, once_gen)) list[append_slot(count)] = v;
 }
 
 __device__ __forceinline__ void stage_init() {
@@ -112,10 +119,6 @@ __device__ __forceinline__ bool grid_barrier(UpdateCtl* c, unsigned& gen, unsign
 // A vertex whose packed word this update changed: the commit compares only these with the stored
 // (distance, parent) (a plain store: every writer stores the same value).
 __device__ __forceinline__ void touch(const SsspParams& p, int v) { p.touch_stamp[v] = p.touch_gen; }
-
-__device__ __forceinline__ bool claim(int* stamp, int v, int generation) {
-  return atomicExch(&stamp[v], generation) != generation;
-}
 
 // The block's minimum into *target with one atomic per block (every thread of the block calls).
 __device__ __forceinline__ void block_min_into(u64 v, u64* target) {
@@ -161,25 +164,28 @@ struct ListSet {
   u64* heavy_cnt;
   int stage_light;
   int stage_med;
+  int* once;      // see staged_append
+  int once_gen;
 };
 
 __device__ __forceinline__ void list_append(const ListSet& L, int v, int len, int heavy_degree) {
   if (len > heavy_degree) {
+    if (L.once && !claim(L.once, v, L.once_gen)) return;
     const u64 chunks = static_cast<u64>((len + kHeavyChunk - 1) / kHeavyChunk);
     const u64 prev = atomicAdd(L.heavy_cnt, (1ULL << 40) | chunks);
     L.heavy[static_cast<int>(prev >> 40)] =
         make_int2(v, static_cast<int>(prev & ((1ULL << 40) - 1)));
   } else if (len > kLightMax) {
-    staged_append(L.stage_med, L.med, L.med_cnt, v);
+    staged_append(L.stage_med, L.med, L.med_cnt, v, L.once, L.once_gen);
   } else {
-    staged_append(L.stage_light, L.light, L.light_cnt, v);
+    staged_append(L.stage_light, L.light, L.light_cnt, v, L.once, L.once_gen);
   }
 }
 
 // A vertex to re-evaluate by the pull pass (classified by in-degree).
 __device__ __forceinline__ void add_candidate(const SsspParams& p, int v) {
   const ListSet L{p.candidates, &p.ctl->cand_count, p.cand_med, &p.ctl->cand_med_count,
-                  p.pull_heavy, &p.ctl->pull_heavy, kStCand, kStCandMed};
+                  p.pull_heavy, &p.ctl->pull_heavy, kStCand, kStCandMed, nullptr, 0};
   list_append(L, v, p.g.in_desc[v].len, p.heavy_degree);
 }
 
@@ -337,7 +343,7 @@ __device__ __forceinline__ void push_commit(const SsspParams& p, Ctx& X, const O
     const bool near = X.pk.dist(r[q].cand) < X.threshold;
     if (near) len[q] = p.g.out_desc[dst].len;
     old[q] = atomicMin(&p.packed[dst], r[q].cand);
-    mark[q] = atomicExch(near ? &p.stamp[dst] : &p.in_far[dst], near ? X.gen : 1);
+    mark[q] = atomicExch(near ? &p.near_stamp[dst] : &p.in_far[dst], near ? X.gen : 1);
   }
 #pragma unroll
   for (int q = 0; q < N; ++q) {
@@ -658,92 +664,197 @@ __device__ __forceinline__ void invalidate(const SsspParams& p, int v) {
   add_candidate(p, v);
 }
 
-// State of the near-far loop carried across a switch between the whole grid and one block.
+// State of the near-far loop (the same in every block).
 struct LoopState {
   int gen;
-  int it;           // push iterations so far (selects the list buffers and counter slots)
-  int iterations;
-  int epochs;
-  int far_parity;   // which of far_a / far_b is the current far pile
-  int done;
-  long long pushes;
+  int it;           // steps of the grid so far (selects the list buffers and counter slots)
+  int iterations;   // push rounds: the steps, and the rounds the blocks ran inside them
+  int epochs;       // threshold raises (select the far pile's buffers and counter slots)
+  bool split_empty; // the last threshold raise brought no vertex below the threshold
   u64 threshold;
 };
 
-constexpr int kSmallFarMax = 4096;
-
-__device__ __forceinline__ void block_barrier() {
-  stage_flush();
-  __threadfence();
-  __syncthreads();
+// A block's own rounds inside one near-far step.  The vertices below the threshold that a block
+// improved wait in its stage; in a step of a short frontier the block pushes them itself, round
+// after round between block barriers, instead of handing them to the next step of the whole grid.
+// Inside one bucket the order of the pushes does not matter for the result (every push is an
+// atomicMin), so no other block has to wait for them; a step of the grid is bound by its barriers
+// and list round trips (8-10 us for a few hundred vertices, 3-4 us for a block's round).  Only
+// frontiers of light rows run this way, up to kLocalShare x the schedule's small-frontier size:
+// longer ones keep every warp busy, and the blocks would push a vertex once for every block
+// that reached it (a 24k-vertex R-MAT frontier measured 1.6x slower).
+constexpr int kLocalLight = 128;    // stage entries a block keeps (more: the grid shares them)
+constexpr int kLocalMed = 8;
+constexpr int kLocalRounds = 1024;  // rounds before the block meets the others again
+constexpr int kLocalShare = 64;
+// Claims of the near list are (round, block) in such a step -- a vertex that a block improves again
+// after it took it, or that another block improves meanwhile, gets a new entry, never a lost
+// one -- and (round, kClaimGrid) otherwise.  What such a step hands on is claimed once more for the
+// whole grid (ListSet::once), so a global list holds a vertex once.
+constexpr int kClaimGrid = kPjMaxBlocks - 1;
+__device__ __forceinline__ int near_claim(int round, int who) {
+  return (round << kClaimBlockBits) | who;
 }
 
-// The near-far loop (fused.cuh:288-417) run by the whole grid (BLOCK = false) or by block 0 alone
-// (BLOCK = true, between block barriers: frontiers of up to `small` vertices do not pay for a grid
-// barrier per step).  Returns 0 when the loop is finished, 1 when the grid should hand over to
-// block 0 (small frontier) or block 0 back to the grid, -1 on a timeout.
-template <bool BLOCK>
-__device__ int near_far(const SsspParams& p, Ctx& X, LoopState& S, unsigned& bar, u64 delta,
-                        long long iteration_cap, int small) {
+// Returns the rounds the block ran; what is left in the stage goes to the global lists.
+__device__ __forceinline__ int local_rounds(const SsspParams& p, Ctx& X, int gen) {
+  __shared__ int s_own[kLocalLight + kLocalMed];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kWarps = kThreads / 32;
+  int round = 0;
+  while (true) {
+    __syncthreads();
+    const int nl = g_stage.cnt[kStNext], nm = g_stage.cnt[kStNextMed];
+    if (nl + nm == 0 || nl > kLocalLight || nm > kLocalMed || round >= kLocalRounds) break;
+    if (static_cast<int>(threadIdx.x) < nl) s_own[threadIdx.x] = g_stage.data[kStNext][threadIdx.x];
+    if (static_cast<int>(threadIdx.x) < nm)
+      s_own[kLocalLight + threadIdx.x] = g_stage.data[kStNextMed][threadIdx.x];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      g_stage.cnt[kStNext] = 0;
+      g_stage.cnt[kStNextMed] = 0;
+      // the blocks waiting at the grid barrier see that this one makes progress
+      if ((round & 63) == 63) atomicAdd(&p.ctl->heartbeat, 1u);
+    }
+    ++round;
+    X.gen = near_claim(gen + round, blockIdx.x);
+    __syncthreads();
+    const int per = (nl + kWarps - 1) / kWarps;
+    static_assert(kLocalLight <= 32 * kWarps && kLocalLight <= kThreads, "one row per lane");
+    if (warp * per < nl) {
+      const int i = warp * per + lane;
+      int owner = -1;
+      u64 du = 0;
+      RowDesc desc{0, 0};
+      if (lane < per && i < nl) {
+        owner = s_own[i];
+        ++X.rows;
+        desc = p.g.out_desc[owner];
+        const u64 word = ld_cg(&p.packed[owner]);
+        if (word != kPackedInf) du = X.pk.dist(word);
+        else desc.len = 0;
+      }
+      warp_rows<kPush>(p, X, owner, du, desc.start, desc.len);
+    }
+    for (int i = warp; i < nm; i += kWarps) {
+      const int owner = s_own[kLocalLight + i];
+      const RowDesc desc = p.g.out_desc[owner];
+      const u64 word = ld_cg(&p.packed[owner]);
+      if (word == kPackedInf) continue;
+      if (lane == 0) ++X.rows;
+      warp_slots<kPush>(p, X, owner, X.pk.dist(word), desc.start, 0, desc.len);
+    }
+  }
+  // the entries that stay: each vertex once for the whole grid
+  const int nl = min(g_stage.cnt[kStNext], kStageCap);
+  const int nm = min(g_stage.cnt[kStNextMed], kStageCap);
+  if (nl + nm == 0) return round;
+  constexpr int kPer = (kStageCap + kThreads - 1) / kThreads;
+  int keep[2][kPer];
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const int i = threadIdx.x + j * kThreads;
+    keep[0][j] = i < nl ? g_stage.data[kStNext][i] : -1;
+    keep[1][j] = i < nm ? g_stage.data[kStNextMed][i] : -1;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    g_stage.cnt[kStNext] = 0;
+    g_stage.cnt[kStNextMed] = 0;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    if (keep[0][j] >= 0 && claim(X.next.once, keep[0][j], X.next.once_gen))
+      staged_append(kStNext, X.next.light, X.next.light_cnt, keep[0][j]);
+    if (keep[1][j] >= 0 && claim(X.next.once, keep[1][j], X.next.once_gen))
+      staged_append(kStNextMed, X.next.med, X.next.med_cnt, keep[1][j]);
+  }
+  return round;
+}
+
+// At step `it` of the near-far loop: the slots of the step after the next start empty.  They were
+// last read at the top of step it - 1 (the rounds: after its barrier, so one slot sooner).
+__device__ __forceinline__ void clear_step(UpdateCtl* c, int it) {
+  const int s = (it + 2) % 3;
+  c->near_cnt[s] = 0;
+  c->near_med_cnt[s] = 0;
+  c->heavy_cnt[s] = 0;
+  c->med_cursor[s] = 0;
+  c->heavy_cursor[s] = 0;
+  c->local_rounds[(it + 1) % 3] = 0;
+}
+
+// The near-far loop (fused.cuh:288-417) run by the whole grid.  Returns false on a timeout.
+__device__ bool near_far(const SsspParams& p, Ctx& X, LoopState& S, unsigned& bar, u64 delta,
+                         long long n, int small) {
   UpdateCtl* c = p.ctl;
-  const long long tid = BLOCK ? threadIdx.x : blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-  const long long threads = BLOCK ? blockDim.x : static_cast<long long>(g_nblk) * blockDim.x;
-  const long long gwarp = tid >> 5;
+  const long long tid = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+  const long long threads = static_cast<long long>(g_nblk) * blockDim.x;
   const long long nwarps = threads >> 5;
-  const bool leader = BLOCK ? threadIdx.x == 0 : tid == 0;
+  const bool leader = tid == 0;
+  const long long step_cap = 4 * n + 64;
   int* lists[2] = {p.near_a, p.near_b};
   int* mlists[2] = {p.near_med_a, p.near_med_b};
   int2* hlists[2] = {p.heavy_a, p.heavy_b};
   const Packing pk = X.pk;
   while (true) {
-    // alone, block 0 shows the waiting blocks that it makes progress (no result is read back)
-    if (BLOCK && threadIdx.x == 0) atomicAdd(&c->heartbeat, 1u);
     const int cs = S.it % 3;
     const int nc = ld_cg(&c->near_cnt[cs]);
     const int mc = ld_cg(&c->near_med_cnt[cs]);
     const u64 hc = ld_cg(&c->heavy_cnt[cs]);
-    const int far_count = ld_cg(&c->far_count);
+    const int fs = S.epochs % 3;
+    const int far_count = ld_cg(&c->far_cnt[fs]);
     const bool near_work = nc > 0 || mc > 0 || (hc >> 40) > 0;
-    const bool fits_block =
-        (hc >> 40) == 0 && nc + mc <= small && (near_work || far_count <= kSmallFarMax);
-    if (!near_work && far_count == 0) return 0;
-    if (small > 0 && (BLOCK ? !fits_block : fits_block)) return 1;
-    int* far = S.far_parity ? p.far_b : p.far_a;
-    int* far2 = S.far_parity ? p.far_a : p.far_b;
+    if (!near_work && far_count == 0) return true;
+    int* far = (S.epochs & 1) ? p.far_b : p.far_a;
     const int step = S.iterations + S.epochs;
-    if (leader && blockIdx.x == 0 && step < 64) {
+    if (leader && step < 64) {
       c->trace_n[step] = near_work ? nc + mc : -far_count;
-      c->trace_h[step] = static_cast<int>(hc & 0xffffffffu) | (BLOCK ? 0x40000000 : 0);
+      c->trace_h[step] = static_cast<int>(hc & 0xffffffffu);
       c->trace_t[step] = static_cast<unsigned>(global_ns() - c->phase_ns[0]);
       c->trace_len = step + 1;
     }
-    if (near_work) {
-      ++S.iterations;
-      if (S.iterations > iteration_cap) {
-        if (leader) atomicOr(&c->error, kErrNotConverged);
-        return 0;
+    if (S.gen > kMaxGeneration - kLocalRounds - 8) {
+      // the claims would run out of generations: start them over
+      for (long long v = tid; v < n; v += threads) {
+        p.near_stamp[v] = 0;
+        p.stamp[v] = 0;
       }
-      S.pushes += nc + mc + static_cast<long long>(hc >> 40);
-      X.gen = ++S.gen;
+      if (!grid_barrier(c, bar)) return false;
+      S.gen = 0;
+      if (leader) c->generations_spent = 1;
+    }
+    if (near_work) {
+      if (S.it > step_cap) {
+        if (leader) atomicOr(&c->error, kErrNotConverged);
+        return true;
+      }
+      ++S.iterations;
+      ++S.gen;
+      const bool local = small > 0 && hc == 0 && mc == 0 &&
+                         nc <= kLocalShare * static_cast<long long>(small);
+      X.gen = near_claim(S.gen, local ? static_cast<int>(blockIdx.x) : kClaimGrid);
       const int nb = (S.it + 1) & 1;
       X.next = ListSet{lists[nb], &c->near_cnt[(S.it + 1) % 3], mlists[nb],
                        &c->near_med_cnt[(S.it + 1) % 3], hlists[nb],
-                       &c->heavy_cnt[(S.it + 1) % 3], kStNext, kStNextMed};
+                       &c->heavy_cnt[(S.it + 1) % 3], kStNext, kStNextMed,
+                       local ? p.stamp : nullptr, S.gen};
       X.far = far;
-      X.far_cnt = &c->far_count;
+      X.far_cnt = &c->far_cnt[fs];
       X.threshold = S.threshold;
-      if (leader) {
-        c->near_cnt[(S.it + 2) % 3] = 0;
-        c->near_med_cnt[(S.it + 2) % 3] = 0;
-        c->heavy_cnt[(S.it + 2) % 3] = 0;
-        c->med_cursor[(S.it + 2) % 3] = 0;
-        c->heavy_cursor[(S.it + 2) % 3] = 0;
-      }
-      const unsigned long long t_busy = (!BLOCK && step == 0) ? global_ns() : 0;
+      S.split_empty = false;
+      if (leader) clear_step(c, S.it);
+      // a step with rounds of the blocks' own deals consecutive entries to different blocks, so that
+      // a short list reaches every SM; otherwise a short list keeps to few blocks, whose warps
+      // share a flush
+      const long long gwarp =
+          local ? static_cast<long long>(threadIdx.x >> 5) * g_nblk + blockIdx.x : tid >> 5;
+      const unsigned long long t_busy = step == 0 ? global_ns() : 0;
       expand<kPush>(p, X, lists[S.it & 1], nc, mlists[S.it & 1], mc, hlists[S.it & 1], hc, gwarp,
-                    nwarps, (!BLOCK && step == 0) ? &c->work[16] : nullptr, &c->med_cursor[cs],
+                    nwarps, step == 0 ? &c->work[16] : nullptr, &c->med_cursor[cs],
                     &c->heavy_cursor[cs]);
-      if (!BLOCK && step == 0) {
+      if (step == 0) {
         // balance of the first step: the slowest warp's and the summed busy time, and warps
         // (met per block in shared memory: one global atomic per block and value)
         __shared__ long long s_busy[2];
@@ -764,46 +875,55 @@ __device__ int near_far(const SsspParams& p, Ctx& X, LoopState& S, unsigned& bar
                     static_cast<unsigned long long>(blockDim.x >> 5));
         }
       }
-      if (BLOCK) block_barrier();
-      else if (!grid_barrier(c, bar)) return -1;
+      if (local) {
+        const int rounds = local_rounds(p, X, S.gen);
+        if (threadIdx.x == 0 && rounds > 0) atomicMax(&c->local_rounds[cs], rounds);
+      }
+      if (!grid_barrier(c, bar)) return false;
+      if (local) {
+        const int most = ld_cg(&c->local_rounds[cs]);
+        S.gen += most;
+        S.iterations += most;
+      }
       ++S.it;
       continue;
     }
-    // near frontier empty: raise the threshold past the far pile
-    ++S.epochs;
-    u64 local = kPackedInf;
-    for (long long i = tid; i < far_count; i += threads) {
-      const u64 word = ld_cg(&p.packed[ld_cg(&far[i])]);
-      if (word != kPackedInf) local = min(local, pk.dist(word));
+    // near frontier empty: raise the threshold by one width and split the far pile.  When the raise
+    // before this one found nothing below its threshold, the smallest distance that it left is
+    // exact (nothing was pushed since) and the threshold skips to it.
+    const u64 before = S.threshold;
+    S.threshold = (S.split_empty ? max(before, ld_cg(&c->far_min[(S.epochs + 2) % 3])) : before) + delta;
+    S.split_empty = true;  // until a push step runs
+    int* rest = (S.epochs & 1) ? p.far_a : p.far_b;
+    // The vertices below go to the lists and slots of the next step: the current slots are what the
+    // blocks that come late still read at the loop's top (no barrier lies in between).
+    if (leader) {
+      c->far_cnt[(S.epochs + 2) % 3] = 0;
+      c->far_min[(S.epochs + 1) % 3] = kPackedInf;
+      clear_step(c, S.it);
     }
-    block_min_into(local, &c->minimum);
-    if (BLOCK) block_barrier();
-    else if (!grid_barrier(c, bar)) return -1;
-    S.threshold = max(S.threshold, ld_cg(reinterpret_cast<const u64*>(&c->minimum))) + delta;
-    ++S.gen;
-    const ListSet now{lists[S.it & 1], &c->near_cnt[cs], mlists[S.it & 1], &c->near_med_cnt[cs],
-                      hlists[S.it & 1], &c->heavy_cnt[cs], kStNext, kStNextMed};
+    const int nb = (S.it + 1) & 1;
+    const ListSet now{lists[nb], &c->near_cnt[(S.it + 1) % 3], mlists[nb],
+                      &c->near_med_cnt[(S.it + 1) % 3], hlists[nb], &c->heavy_cnt[(S.it + 1) % 3],
+                      kStNext, kStNextMed, nullptr, 0};
+    u64 left = kPackedInf;
     for (long long i = tid; i < far_count; i += threads) {
       const int v = ld_cg(&far[i]);
       const u64 word = ld_cg(&p.packed[v]);
       const u64 d = word == kPackedInf ? kPackedInf : pk.dist(word);
       if (d < S.threshold) {
         p.in_far[v] = 0;
-        if (claim(p.stamp, v, S.gen)) list_append(now, v, p.g.out_desc[v].len, p.heavy_degree);
+        // a vertex that fell below the old threshold since joined a near list then
+        if (d >= before) list_append(now, v, p.g.out_desc[v].len, p.heavy_degree);
       } else {
-        staged_append(kStFar, far2, &c->far2_count, v);
+        left = min(left, d);
+        staged_append(kStFar, rest, &c->far_cnt[(S.epochs + 1) % 3], v);
       }
     }
-    if (BLOCK) block_barrier();
-    else if (!grid_barrier(c, bar)) return -1;
-    if (leader) {
-      c->far_count = ld_cg(&c->far2_count);
-      c->far2_count = 0;
-      c->minimum = kPackedInf;
-    }
-    if (BLOCK) block_barrier();
-    else if (!grid_barrier(c, bar)) return -1;
-    S.far_parity ^= 1;
+    block_min_into(left, &c->far_min[fs]);
+    if (!grid_barrier(c, bar)) return false;
+    ++S.epochs;
+    ++S.it;
   }
 }
 
@@ -902,7 +1022,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
           changed = 2;
           if (p.walk) {
             const ListSet W0{p.near_a, &c->walk_cnt[0], p.near_med_a, &c->walk_med_cnt[0],
-                             p.heavy_a, &c->walk_heavy[0], kStNext, kStNextMed};
+                             p.heavy_a, &c->walk_heavy[0], kStNext, kStNextMed, nullptr, 0};
             list_append(W0, v, p.g.out_desc[v].len, p.heavy_degree);
           }
         }
@@ -1121,7 +1241,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
         X.next = ListSet{nb ? p.near_b : p.near_a, &c->walk_cnt[(level + 1) % 3],
                          nb ? p.near_med_b : p.near_med_a, &c->walk_med_cnt[(level + 1) % 3],
                          nb ? p.heavy_b : p.heavy_a, &c->walk_heavy[(level + 1) % 3], kStNext,
-                         kStNextMed};
+                         kStNextMed, nullptr, 0};
         if (tid == 0) {
           c->walk_cnt[(level + 2) % 3] = 0;
           c->walk_med_cnt[(level + 2) % 3] = 0;
@@ -1181,7 +1301,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
       Ctx Y = X;
       Y.gen = gen_pull;
       Y.next = ListSet{p.frontier, &c->frontier_count, nullptr, nullptr, nullptr, nullptr, kStNext,
-                       kStNextMed};
+                       kStNextMed, nullptr, 0};
       Y.slots = Y.words = Y.atomics = Y.appends = Y.rows = Y.tries = 0;
       expand<kPull>(p, Y, p.candidates, ld_cg(&c->cand_count), p.cand_med,
                     ld_cg(&c->cand_med_count), p.pull_heavy, ld_cg(&c->pull_heavy), gwarp, nwarps);
@@ -1207,64 +1327,25 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
   if (!grid_barrier(c, bar)) return;
   const u64 smallest = ld_cg(reinterpret_cast<const u64*>(&c->minimum));
   X.threshold = (smallest == kPackedInf ? 0 : smallest) + delta;
-  int* lists[2] = {p.near_a, p.near_b};
-  int* mlists[2] = {p.near_med_a, p.near_med_b};
-  int2* hlists[2] = {p.heavy_a, p.heavy_b};
-  int* far = p.far_a;
-  X.far_cnt = &c->far_count;
-  ++gen;
+  X.far_cnt = &c->far_cnt[0];
+  if (tid < 3) c->far_min[tid] = kPackedInf;
   for (long long i = tid; i < frontier_count; i += threads) {
     const int v = ld_cg(&p.frontier[i]);
     const u64 word = ld_cg(&p.packed[v]);
     const u64 d = word == kPackedInf ? kPackedInf : pk.dist(word);
     if (d < X.threshold) {
-      if (claim(p.stamp, v, gen))
-        list_append(ListSet{lists[0], &c->near_cnt[0], mlists[0], &c->near_med_cnt[0], hlists[0],
-                            &c->heavy_cnt[0], kStNext, kStNextMed},
-                    v, p.g.out_desc[v].len, p.heavy_degree);
+      list_append(ListSet{p.near_a, &c->near_cnt[0], p.near_med_a, &c->near_med_cnt[0], p.heavy_a,
+                          &c->heavy_cnt[0], kStNext, kStNextMed, nullptr, 0},
+                  v, p.g.out_desc[v].len, p.heavy_degree);
     } else if (atomicExch(&p.in_far[v], 1) == 0) {
-      staged_append(kStFar, far, &c->far_count, v);
+      staged_append(kStFar, p.far_a, &c->far_cnt[0], v);
     }
   }
   if (!grid_barrier(c, bar)) return;
-  if (tid == 0) c->minimum = kPackedInf;
-  if (!grid_barrier(c, bar)) return;
-  LoopState S{gen, 0, 0, 0, 0, 0, 0, X.threshold};
-  const long long iteration_cap = 4 * n + 64;
-  const int small = p.small_frontier;
-  while (true) {
-    const int r = near_far<false>(p, X, S, bar, delta, iteration_cap, small);
-    if (r < 0) return;
-    if (r == 0) break;
-    // a small frontier: block 0 runs the loop alone while the other blocks wait at one barrier
-    if (blockIdx.x == 0) {
-      const int rb = near_far<true>(p, X, S, bar, delta, iteration_cap, small);
-      if (threadIdx.x == 0) {
-        S.done = rb == 0 ? 1 : 0;
-        c->loop_state[0] = S.gen;
-        c->loop_state[1] = S.it;
-        c->loop_state[2] = S.iterations;
-        c->loop_state[3] = S.epochs;
-        c->loop_state[4] = S.far_parity;
-        c->loop_state[5] = S.done;
-        c->loop_pushes = S.pushes;
-        c->loop_threshold = S.threshold;
-      }
-    }
-    if (!grid_barrier(c, bar)) return;
-    S.gen = ld_cg(&c->loop_state[0]);
-    S.it = ld_cg(&c->loop_state[1]);
-    S.iterations = ld_cg(&c->loop_state[2]);
-    S.epochs = ld_cg(&c->loop_state[3]);
-    S.far_parity = ld_cg(&c->loop_state[4]);
-    S.done = ld_cg(&c->loop_state[5]);
-    S.pushes = ld_cg(&c->loop_pushes);
-    S.threshold = ld_cg(&c->loop_threshold);
-    if (S.done) break;
-  }
+  LoopState S{gen, 0, 0, 0, false, X.threshold};
+  if (!near_far(p, X, S, bar, delta, n, p.small_frontier)) return;
   gen = S.gen;
   const int iterations = S.iterations, epochs = S.epochs;
-  const long long pushes = S.pushes;
   if (tid == 0) c->phase_ns[6] = global_ns();
 
   // ---- commit: unpack (fused.cuh:419-494) ------------------------------------------------------
@@ -1367,6 +1448,11 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
     red_sum(red, 16, walk_rows);
     red_sum(red, 17, walk_slots);
     __syncthreads();
+    if (threadIdx.x == 18) {
+      const long long t = red_total(red, 6);
+      if (t != 0)
+        atomicAdd(reinterpret_cast<unsigned long long*>(&c->pushes), static_cast<unsigned long long>(t));
+    }
     if (threadIdx.x < 18) {
       // reduction slot -> work counter (slot 0: affected)
       const int w = threadIdx.x < 10 ? static_cast<int>(threadIdx.x) - 1 + (threadIdx.x >= 3 ? 1 : 0)
@@ -1382,8 +1468,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
     c->phase_ns[7] = global_ns();
     c->iterations = iterations;
     c->epochs = epochs;
-    c->pushes = pushes;
-    c->last_generation = gen;
+    c->last_generation = ld_cg(&c->generations_spent) ? kMaxGeneration : gen;
     if (p.hist) {
       TreeHistory h{};
       h.invalidated = ld_cg(&c->invalidated);
@@ -1439,7 +1524,7 @@ int update_blocks_per_sm(Context& ctx) {
     expects(per_sm >= 1, "sssp: the persistent kernel does not fit on an SM", DYNGB200_NOT_SUPPORTED);
     ctx.update_blocks_per_sm = per_sm;
   }
-  expects(ctx.update_blocks_per_sm * ctx.sm_count <= kPjMaxBlocks,
+  expects(ctx.update_blocks_per_sm * ctx.sm_count < kPjMaxBlocks,
           "sssp: more persistent blocks than the pointer-jumping lists support", DYNGB200_NOT_SUPPORTED);
   return ctx.update_blocks_per_sm;
 }
@@ -1511,7 +1596,7 @@ static SsspParams base_params(Context& ctx, Graph& g, Tree& t) {
   p.packed = t.packed.ptr;
   p.stamp = ws.stamp.ptr;
   p.touch_stamp = ws.touch_stamp.ptr;
-  p.flag = ws.flag.ptr;
+  p.near_stamp = ws.near_stamp.ptr;
   p.in_far = ws.in_far.ptr;
   p.ancestor = ws.ancestor.ptr;
   p.candidates = ws.candidates.ptr;
@@ -2173,7 +2258,7 @@ void sssp_compute_static(Graph& g, int32_t source, int objective, long long delt
   p.stamp = ints + 0 * N;
   p.touch_stamp = ints + 1 * N;
   p.in_far = ints + 2 * N;
-  p.flag = ints + 3 * N;
+  p.near_stamp = ints + 3 * N;
   p.ancestor = ints + 4 * N;
   p.candidates = ints + 5 * N;
   p.frontier = ints + 6 * N;
@@ -2198,7 +2283,7 @@ void sssp_compute_static(Graph& g, int32_t source, int objective, long long delt
   p.tree_bits = pk.bits;
   p.tree_n = n;
   // the array keeps the previous call's contents: stamps and far marks must start at zero
-  DYNGB200_CUDA(cudaMemsetAsync(ints, 0, 3 * N * sizeof(int), s));
+  DYNGB200_CUDA(cudaMemsetAsync(ints, 0, 4 * N * sizeof(int), s));
   UpdateCtl init{};
   init.err_index = INT64_MAX;
   init.n_old = n;

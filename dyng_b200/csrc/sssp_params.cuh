@@ -31,7 +31,7 @@ struct SsspParams {
   // scratch
   int* stamp;
   int* touch_stamp;
-  int* flag;
+  int* near_stamp;       // claims of the fused kernel's near-far loop
   int* in_far;
   int* ancestor;
   int* candidates;
@@ -51,7 +51,7 @@ struct SsspParams {
   int touch_gen;
   int heavy_degree;
   long long delta_override;
-  int small_frontier;    // frontiers up to this size run on block 0 alone (0: never)
+  int small_frontier;    // short near frontiers stay with the blocks that found them (0: never)
   UpdateCtl* ctl;
   TreeHistory* hist;
   int* pj_blk;           // survivor counts of the pointer-jumping rounds: 2 x kPjMaxBlocks

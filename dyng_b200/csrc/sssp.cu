@@ -88,6 +88,10 @@ __device__ __forceinline__ void stage_init() {
 // Copy every non-empty stage to its global list (all threads of the block).
 __device__ __forceinline__ void stage_flush() {
   __syncthreads();
+  int any = 0;
+#pragma unroll
+  for (int id = 0; id < kStages; ++id) any |= g_stage.cnt[id];
+  if (any == 0) return;  // every thread reads the same counts, and none appends before a barrier
   if (threadIdx.x < kStages) {
     const int id = threadIdx.x;
     const int n = min(g_stage.cnt[id], kStageCap);
@@ -194,6 +198,7 @@ struct Ctx {
   Packing pk;
   u64 maxd;
   u64 threshold;
+  u64 low;       // pull: the smallest distance an offer of this thread brought into the frontier
   int gen;       // claim generation of the appends
   ListSet next;  // push: next near frontier; walk: next level; pull: the frontier (light only)
   int* far;
@@ -289,6 +294,7 @@ __device__ __forceinline__ void offer_owner(const SsspParams& p, Ctx& X, int own
   if (cand < old) {
     ++X.atomics;
     touch(p, owner);
+    X.low = min(X.low, X.pk.dist(cand));
   }
   if (claimed) {
     ++X.appends;
@@ -959,11 +965,11 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
   X.pk.no_parent = X.pk.bits ? (1ULL << X.pk.bits) - 1 : 0;
   X.maxd = c->max_distance;
   X.threshold = 0;
+  X.low = kPackedInf;
   X.slots = X.words = X.atomics = X.appends = X.rows = X.tries = 0;
   const Packing pk = X.pk;
   const u64 delta = static_cast<u64>(p.delta_override > 0 ? p.delta_override : c->delta);
   int gen = p.generation;
-  int frontier_count = 0;
   // work counters (see dyngb200_stats::work)
   long long w_visits = 0, w_jumps = 0, w_inval = 0;
   unsigned pull_slots = 0, pull_words = 0, pull_rows = 0, unpacked = 0;
@@ -973,9 +979,15 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
   if (p.from_scratch) {
     for (long long v = tid; v < n; v += threads)
       p.packed[v] = v == p.source ? pk.pack(0, -1) : kPackedInf;
-    if (tid == 0) p.frontier[0] = p.source;
-    frontier_count = 1;
+    // the source is the whole frontier, at distance 0
+    if (tid == 0)
+      list_append(ListSet{p.near_a, &c->near_cnt[0], p.near_med_a, &c->near_med_cnt[0], p.heavy_a,
+                          &c->heavy_cnt[0], kStNext, kStNextMed, nullptr, 0},
+                  p.source, p.g.out_desc[p.source].len, p.heavy_degree);
+    X.threshold = delta;
+    if (tid < 3) c->far_min[tid] = kPackedInf;
     if (!grid_barrier(c, bar)) return;
+    if (tid == 0) c->phase_ns[5] = global_ns();
   } else {
     const int gen_inv = ++gen;
     const int gen_pull = ++gen;
@@ -1262,9 +1274,13 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
         c->phase_ns[2] = global_ns();
       }
     }
-    if (!grid_barrier(c, bar)) return;
-    if (tid == 0) c->phase_ns[3] = global_ns();
+    // The lists and stamps of the invalidation are complete (its last step ended in a barrier).
     // ---- insertion heads: pulled, or (canonical trees) offered the inserted edge ----------------
+    // The offers of a canonical tree's heads need no barrier before the pull: both only lower words
+    // by atomicMin towards the same fixed point.  A head whose tail is invalidated and not pulled
+    // yet gets no offer here; the tail joins the frontier with its pull and is pushed over the
+    // inserted edge then.
+    if (tid == 0) c->phase_ns[3] = c->phase_ns[2];
     for (long long i = tid; i < pairs; i += threads) {
       ++pair_visits;
       const int slot = p.pair_list[i];
@@ -1289,12 +1305,15 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
       const u64 cand = pk.pack(nd, u);
       if (cand >= ld_cg(&p.packed[v])) continue;
       const u64 old = atomicMin(&p.packed[v], cand);
-      if (cand < old) touch(p, v);
+      if (cand < old) {
+        touch(p, v);
+        X.low = min(X.low, nd);
+      }
       if (nd < pk.dist(old) && claim(p.stamp, v, gen_pull))
         staged_append(kStNext, p.frontier, &c->frontier_count, v);
     }
     block_sum_into(w_inval, &c->invalidated);
-    if (!grid_barrier(c, bar)) return;
+    if (!p.offer_heads && !grid_barrier(c, bar)) return;
     if (tid == 0) c->phase_ns[4] = global_ns();
     // ---- pull pass (fused.cuh:258-285): every candidate takes its best in-neighbour ----------
     {
@@ -1311,37 +1330,33 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
       pull_atomics = Y.atomics;
       pull_appends = Y.appends;
       X.tries += Y.tries;
+      // the frontier's smallest distance: every word in it was brought by one of these offers
+      block_min_into(Y.low, &c->minimum);
     }
     if (!grid_barrier(c, bar)) return;
-    frontier_count = ld_cg(&c->frontier_count);
+    const int frontier_count = ld_cg(&c->frontier_count);
+    if (tid == 0) c->phase_ns[5] = global_ns();
+    // the first split of the near-far loop, at one width past the smallest distance
+    const u64 smallest = ld_cg(reinterpret_cast<const u64*>(&c->minimum));
+    X.threshold = (smallest == kPackedInf ? 0 : smallest) + delta;
+    if (tid < 3) c->far_min[tid] = kPackedInf;
+    for (long long i = tid; i < frontier_count; i += threads) {
+      const int v = ld_cg(&p.frontier[i]);
+      const u64 word = ld_cg(&p.packed[v]);
+      const u64 d = word == kPackedInf ? kPackedInf : pk.dist(word);
+      if (d < X.threshold) {
+        list_append(ListSet{p.near_a, &c->near_cnt[0], p.near_med_a, &c->near_med_cnt[0], p.heavy_a,
+                            &c->heavy_cnt[0], kStNext, kStNextMed, nullptr, 0},
+                    v, p.g.out_desc[v].len, p.heavy_degree);
+      } else if (atomicExch(&p.in_far[v], 1) == 0) {
+        staged_append(kStFar, p.far_a, &c->far_cnt[0], v);
+      }
+    }
+    if (!grid_barrier(c, bar)) return;
   }
-  if (tid == 0) c->phase_ns[5] = global_ns();
 
   // ---- near-far propagation (fused.cuh:288-417) ------------------------------------------------
-  u64 local = kPackedInf;
-  for (long long i = tid; i < frontier_count; i += threads) {
-    const u64 word = ld_cg(&p.packed[ld_cg(&p.frontier[i])]);
-    if (word != kPackedInf) local = min(local, pk.dist(word));
-  }
-  block_min_into(local, &c->minimum);
-  if (!grid_barrier(c, bar)) return;
-  const u64 smallest = ld_cg(reinterpret_cast<const u64*>(&c->minimum));
-  X.threshold = (smallest == kPackedInf ? 0 : smallest) + delta;
-  X.far_cnt = &c->far_cnt[0];
-  if (tid < 3) c->far_min[tid] = kPackedInf;
-  for (long long i = tid; i < frontier_count; i += threads) {
-    const int v = ld_cg(&p.frontier[i]);
-    const u64 word = ld_cg(&p.packed[v]);
-    const u64 d = word == kPackedInf ? kPackedInf : pk.dist(word);
-    if (d < X.threshold) {
-      list_append(ListSet{p.near_a, &c->near_cnt[0], p.near_med_a, &c->near_med_cnt[0], p.heavy_a,
-                          &c->heavy_cnt[0], kStNext, kStNextMed, nullptr, 0},
-                  v, p.g.out_desc[v].len, p.heavy_degree);
-    } else if (atomicExch(&p.in_far[v], 1) == 0) {
-      staged_append(kStFar, p.far_a, &c->far_cnt[0], v);
-    }
-  }
-  if (!grid_barrier(c, bar)) return;
+  ++gen;
   LoopState S{gen, 0, 0, 0, false, X.threshold};
   if (!near_far(p, X, S, bar, delta, n, p.small_frontier)) return;
   gen = S.gen;

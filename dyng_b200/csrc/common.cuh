@@ -51,6 +51,14 @@ struct GraphCounters {
   long long idx_live, idx_dead; // edge index: live keys and deleted markers
 };
 
+// One entry of the edge index: the key (u << 32 | v) and the edge's absolute slots in the out and
+// in arenas, in one 16-byte record, so that a probe brings the slots with the key (one 32-byte
+// sector per lookup; with the three in arrays of their own a lookup cost three).
+struct alignas(16) EdgeSlot {
+  unsigned long long key;
+  unsigned out, in;
+};
+
 // The device view of one slack-row graph (out-rows plus the in-edge mirror).
 struct GraphView {
   RowDesc* out_desc;
@@ -70,11 +78,9 @@ struct GraphView {
   int allow_multi;  // multi_edges::allow
   GraphCounters* counters;
   ColumnStats* columns;  // k entries
-  // Edge index (simple graphs): open addressing on (u << 32 | v) -> absolute slot of the edge in
-  // the out arena and in the in arena.  emask + 1 entries; empty keys ~0, deleted ~0 - 1.
-  unsigned long long* ekey;
-  unsigned* eout;
-  unsigned* ein;
+  // Edge index (simple graphs): open addressing on (u << 32 | v).  emask + 1 entries; empty keys
+  // ~0, deleted ~0 - 1.
+  EdgeSlot* eidx;
   long long emask;
 };
 
@@ -150,13 +156,18 @@ __device__ __forceinline__ u64 edge_key(int32_t u, int32_t v) {
   return (static_cast<u64>(static_cast<uint32_t>(u)) << 32) | static_cast<uint32_t>(v);
 }
 
-// Slot of a live key in the edge index, or -1.
-__device__ __forceinline__ long long index_find(const GraphView& g, u64 key) {
+// Slot of a live key in the edge index, or -1; *entry (optional) receives the entry.
+__device__ __forceinline__ long long index_find(const GraphView& g, u64 key,
+                                                EdgeSlot* entry = nullptr) {
   long long h = static_cast<long long>(mix64(key) & static_cast<u64>(g.emask));
   for (long long probe = 0; probe <= g.emask; ++probe) {
-    const u64 cur = g.ekey[h];
-    if (cur == key) return h;
-    if (cur == kKeyEmpty) return -1;
+    const ulonglong2 raw = __ldcg(reinterpret_cast<const ulonglong2*>(&g.eidx[h]));
+    if (raw.x == key) {
+      if (entry)
+        *entry = EdgeSlot{raw.x, static_cast<unsigned>(raw.y), static_cast<unsigned>(raw.y >> 32)};
+      return h;
+    }
+    if (raw.x == kKeyEmpty) return -1;
     h = (h + 1) & g.emask;
   }
   return -1;
@@ -167,9 +178,9 @@ __device__ __forceinline__ long long index_find(const GraphView& g, u64 key) {
 __device__ __forceinline__ long long index_insert(const GraphView& g, u64 key, bool* reused) {
   long long h = static_cast<long long>(mix64(key) & static_cast<u64>(g.emask));
   for (long long probe = 0; probe <= g.emask; ++probe) {
-    u64 cur = g.ekey[h];
+    u64 cur = __ldcg(&g.eidx[h].key);
     while (cur == kKeyEmpty || cur == kKeyDeleted) {
-      const u64 prev = atomicCAS(&g.ekey[h], cur, key);
+      const u64 prev = atomicCAS(&g.eidx[h].key, cur, key);
       if (prev == cur) {
         *reused = cur == kKeyDeleted;
         return h;
@@ -189,7 +200,7 @@ __device__ __forceinline__ long long index_find_or_insert(const GraphView& g, u6
   long long h = static_cast<long long>(mix64(key) & static_cast<u64>(g.emask));
   long long first_deleted = -1;
   for (long long probe = 0; probe <= g.emask; ++probe) {
-    const u64 cur = g.ekey[h];
+    const u64 cur = __ldcg(&g.eidx[h].key);
     if (cur == key) {
       *inserted = false;
       return h;
@@ -199,7 +210,7 @@ __device__ __forceinline__ long long index_find_or_insert(const GraphView& g, u6
     h = (h + 1) & g.emask;
   }
   // not in the index: claim the first deleted slot seen, else insert from scratch
-  if (first_deleted >= 0 && atomicCAS(&g.ekey[first_deleted], kKeyDeleted, key) == kKeyDeleted) {
+  if (first_deleted >= 0 && atomicCAS(&g.eidx[first_deleted].key, kKeyDeleted, key) == kKeyDeleted) {
     *inserted = true;
     *reused = true;
     return first_deleted;

@@ -420,10 +420,11 @@ __device__ void ph_match(const ApplyParams& p, long long tid, long long threads)
   const int pairs = c->pairs;
   for (long long i = tid; i < pairs; i += threads) {
     const int slot = p.list[i];
-    const long long e = index_find(p.g, p.key[slot]);
+    EdgeSlot at;
+    const long long e = index_find(p.g, p.key[slot], &at);
     if (e >= 0) {
-      p.out_pos[slot] = static_cast<int>(p.g.eout[e]);
-      p.in_pos[slot] = static_cast<int>(p.g.ein[e]);
+      p.out_pos[slot] = static_cast<int>(at.out);
+      p.in_pos[slot] = static_cast<int>(at.in);
       p.out_count[slot] = 1;
       p.in_count[slot] = 1;
     }
@@ -791,7 +792,7 @@ __device__ void ph_mutate(const ApplyParams& p, BlockRed& R, long long tid, long
       }
       if (tomb && !(flags & kPairAppend)) {
         // the edge is gone: its index key becomes a deleted marker
-        p.g.ekey[p.in_pos2[slot]] = kKeyDeleted;
+        p.g.eidx[p.in_pos2[slot]].key = kKeyDeleted;
         ++idx_deleted;
       }
       continue;
@@ -889,7 +890,7 @@ __device__ void ph_move(const ApplyParams& p, long long tid, long long threads) 
             w[j * p.g.arena_cap + dst + pos] = w[j * p.g.arena_cap + desc.start + e];
           if (!p.g.allow_multi) {
             const long long ie = index_find(p.g, side == 0 ? edge_key(r, x) : edge_key(x, r));
-            if (ie >= 0) (side == 0 ? p.g.eout : p.g.ein)[ie] = dst + pos;
+            if (ie >= 0) *(side == 0 ? &p.g.eidx[ie].out : &p.g.eidx[ie].in) = dst + pos;
             else set_error(&c->error, kErrInternal);
           }
         }
@@ -939,8 +940,7 @@ __device__ void ph_append(const ApplyParams& p, BlockRed& R, long long tid, long
         ++idx_new;
         idx_reused += reused ? 1 : 0;
       }
-      p.g.eout[ie] = placed[0];
-      p.g.ein[ie] = placed[1];
+      *reinterpret_cast<uint2*>(&p.g.eidx[ie].out) = make_uint2(placed[0], placed[1]);
     }
   }
   acc_stage(R, acc, 0);
@@ -1179,7 +1179,7 @@ __global__ void k_insert_flags(ApplyParams p, unsigned char* out) {
 __global__ void k_index_clear(GraphView g) {
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i <= g.emask;
        i += static_cast<long long>(gridDim.x) * blockDim.x)
-    g.ekey[i] = kKeyEmpty;
+    g.eidx[i].key = kKeyEmpty;
 }
 
 // One warp per row, the lanes over its slots: hub rows (tens of thousands of slots in R-MAT
@@ -1200,7 +1200,7 @@ __global__ void k_index_out(GraphView g, long long n, unsigned* error) {
         atomicOr(error, kErrCapacity);  // a full table: the build fails, no other walk needed
         return;
       }
-      g.eout[ie] = d.start + e;
+      g.eidx[ie].out = d.start + e;
       ++live;
     }
   }
@@ -1222,7 +1222,7 @@ __global__ void k_index_in(GraphView g, long long n, unsigned* error) {
         atomicOr(error, kErrInternal);
         return;
       }
-      g.ein[ie] = d.start + e;
+      g.eidx[ie].in = d.start + e;
     }
   }
 }
@@ -1837,15 +1837,10 @@ void graph_index_build(Context& ctx, Graph& g, long long extra, long long min_ca
   ws.ctl.reserve(1, s);  // before the index changes: every allocation comes first
   const long long want = index_want(g, extra, min_cap);
   if (want != g.ecap) {
-    // the new arrays first: a failed allocation leaves the old index, whole, in place
-    DevBuf<u64> key;
-    DevBuf<unsigned> out, in;
-    key.reserve(static_cast<size_t>(want));
-    out.reserve(static_cast<size_t>(want));
-    in.reserve(static_cast<size_t>(want));
-    g.ekey.swap(key);
-    g.eout.swap(out);
-    g.ein.swap(in);
+    // the new array first: a failed allocation leaves the old index, whole, in place
+    DevBuf<EdgeSlot> fresh;
+    fresh.reserve(static_cast<size_t>(want));
+    g.eidx.swap(fresh);
     g.ecap = want;
   }
   GraphCounters gc = g.host_counters;
@@ -2016,13 +2011,8 @@ void graph_compact(Context& ctx, Graph& g, long long need_out, long long need_in
   // control block are allocated now, so the rebuild cannot fail on an allocation after the
   // slots moved (the old index would point at other edges' slots)
   const long long index_cap = g.props.allow_multi ? g.ecap : index_want(g, 0, g.ecap);
-  DevBuf<u64> ikey;
-  DevBuf<unsigned> iout, iin;
-  if (index_cap != g.ecap) {
-    ikey.reserve(static_cast<size_t>(index_cap));
-    iout.reserve(static_cast<size_t>(index_cap));
-    iin.reserve(static_cast<size_t>(index_cap));
-  }
+  DevBuf<EdgeSlot> index;
+  if (index_cap != g.ecap) index.reserve(static_cast<size_t>(index_cap));
   ctx.ws.ctl.reserve(1, s);
   for (int side = 0; side < 2; ++side) {
     DevBuf<int32_t>& col = side == 0 ? g.out_col : g.in_col;
@@ -2047,9 +2037,7 @@ void graph_compact(Context& ctx, Graph& g, long long need_out, long long need_in
   g.in_w.swap(nw[1]);
   g.arena_cap = arena;
   if (index_cap != g.ecap) {
-    g.ekey.swap(ikey);
-    g.eout.swap(iout);
-    g.ein.swap(iin);
+    g.eidx.swap(index);
     g.ecap = index_cap;
   }
   ++g.compactions;
@@ -2384,9 +2372,7 @@ void graph_copy(Context& ctx, Graph& dst, const Graph& src) {
   copy_buf(dst.in_w, src.in_w, s);
   copy_buf(dst.counters, src.counters, s);
   copy_buf(dst.columns, src.columns, s);
-  copy_buf(dst.ekey, src.ekey, s);
-  copy_buf(dst.eout, src.eout, s);
-  copy_buf(dst.ein, src.ein, s);
+  copy_buf(dst.eidx, src.eidx, s);
   dst.version = src.version;
   dst.props = src.props;
   dst.k = src.k;

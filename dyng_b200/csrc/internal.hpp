@@ -305,8 +305,7 @@ struct Graph {
   DevBuf<int32_t> out_w, in_w;
   DevBuf<GraphCounters> counters;
   DevBuf<ColumnStats> columns;
-  DevBuf<u64> ekey;  // edge index (simple graphs)
-  DevBuf<unsigned> eout, ein;
+  DevBuf<EdgeSlot> eidx;  // edge index (simple graphs)
   long long ecap = 0;
   GraphCounters host_counters{};
   std::vector<ColumnStats> host_columns;
@@ -337,9 +336,7 @@ struct Graph {
     v.allow_multi = props.allow_multi;
     v.counters = counters.ptr;
     v.columns = columns.ptr;
-    v.ekey = ekey.ptr;
-    v.eout = eout.ptr;
-    v.ein = ein.ptr;
+    v.eidx = eidx.ptr;
     v.emask = ecap - 1;
     return v;
   }

@@ -182,8 +182,8 @@ __global__ void k_mosp_first_index(GraphView g, long long n, const int32_t* cpar
        v += static_cast<long long>(gridDim.x) * blockDim.x) {
     const int32_t p = cpar[v];
     if (p < 0 || v == source) continue;
-    const long long ie = index_find(g, edge_key(p, static_cast<int32_t>(v)));
-    if (ie >= 0) first[v] = g.eout[ie];
+    EdgeSlot at;
+    if (index_find(g, edge_key(p, static_cast<int32_t>(v)), &at) >= 0) first[v] = at.out;
   }
 }
 

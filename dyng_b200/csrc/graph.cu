@@ -105,6 +105,9 @@ struct ApplyParams {
   int* new_cap_in;
   int* live_out;
   int* live_in;
+  // long relocated rows: (touched row, first chunk), and the live slots of every chunk
+  int2* move_list;
+  int* move_live;
   // column statistics deltas (k entries each)
   long long* col_sum_delta;
   long long* col_removed_at_max;
@@ -605,6 +608,11 @@ __device__ __forceinline__ u64 warp_reserve(u64 amount, u64* counter) {
   return base + incl - amount;
 }
 
+// A relocated row of more slots than this moves in chunks spread over the grid's warps.  One warp
+// moved a row of 50,000 slots in 0.4 ms while the others waited: at R-MAT scale 20 with 75k edges
+// re-inserted into their old (mostly long) rows the step took 540 us, 20 us of it for the rest.
+constexpr unsigned kMoveChunk = 512;
+
 // ---- F: per touched row: stay in place or move to the top of the arena -------------------------
 // A row that overflows its slack (or is mostly tombstones) gets a new place at the arena top.  The warps iterate together so that the arena
 // space of a warp's relocated rows is reserved with one atomic per side.
@@ -653,6 +661,11 @@ __device__ void ph_alloc(const ApplyParams& p, BlockRed& R, long long tid, long 
       moved_in += n_in;
     }
     if (!active) continue;
+    if (reloc && tail - start > kMoveChunk) {
+      const u64 chunks = (tail - start + kMoveChunk - 1) / kMoveChunk;
+      const u64 prev = atomicAdd(&c->move_heavy, (1ULL << 40) | chunks);
+      p.move_list[prev >> 40] = make_int2(i, static_cast<int>(prev & ((1ULL << 40) - 1)));
+    }
     if (reloc) {
       const u64 at = side == 0 ? at_out : at_in;
       if (at + new_cap > static_cast<u64>(p.g.arena_cap) || at + new_cap > 0xffffffffULL) {
@@ -844,11 +857,77 @@ __device__ void ph_mutate(const ApplyParams& p, BlockRed& R, long long tid, long
 }
 
 // ---- H: move relocated rows (live slots, in order) ---------------------------------------------
+// Which touched row a chunk of a long relocated row belongs to: the last entry whose first chunk
+// is not past it (a 32-ary search by the warp; the entries' first chunks grow with their index).
+__device__ __forceinline__ int2 find_move(const ApplyParams& p, int count, int ch) {
+  const int lane = threadIdx.x & 31;
+  int lo = 0, hi = count;
+  while (hi - lo > 1) {
+    const int stride = (hi - lo + 31) >> 5;
+    const int probe = lo + lane * stride;
+    const bool ok = probe < hi && __ldcg(&p.move_list[probe].y) <= ch;
+    const int last = 31 - __clz(__ballot_sync(0xffffffffu, ok));  // lane 0: list[lo].y <= ch
+    lo = lo + last * stride;
+    hi = min(hi, lo + stride);
+  }
+  return make_int2(__ldcg(&p.move_list[lo].x), __ldcg(&p.move_list[lo].y));
+}
+
+// The live slots of every chunk of the long relocated rows (after the tombstones of step G): each
+// chunk's place in the new row is the sum of the chunks before it.
+__device__ void ph_move_count(const ApplyParams& p, long long tid, long long threads) {
+  UpdateCtl* c = p.ctl;
+  const int lane = threadIdx.x & 31;
+  const int count = static_cast<int>(c->move_heavy >> 40);
+  const int chunks = static_cast<int>(c->move_heavy & ((1ULL << 40) - 1));
+  const int rows_out = c->rows_out;
+  for (long long ch = tid >> 5; ch < chunks; ch += threads >> 5) {
+    const int2 at = find_move(p, count, static_cast<int>(ch));
+    const int side = at.x < rows_out ? 0 : 1;
+    const int s = side == 0 ? at.x : at.x - rows_out;
+    const RowDesc desc = (side == 0 ? p.g.out_desc : p.g.in_desc)[(side == 0 ? p.rows_out : p.rows_in)[s]];
+    const int32_t* col = (side == 0 ? p.g.out_col : p.g.in_col) + desc.start;
+    const int e0 = static_cast<int>(ch - at.y) * static_cast<int>(kMoveChunk);
+    const int e1 = min(desc.len, e0 + static_cast<int>(kMoveChunk));
+    int live = 0;
+    for (int e = e0 + lane; e < e1; e += 32) live += __ldcg(&col[e]) >= 0;
+    live = __reduce_add_sync(0xffffffffu, live);
+    if (lane == 0) p.move_live[ch] = live;
+  }
+}
+
+// Slots [e0, e1) of touched row (side, s) to its new place, whose first `written` slots are taken,
+// by one warp; the edge index follows.  Every lane moves one slot per step.
+__device__ __forceinline__ void move_slots(const ApplyParams& p, int side, int32_t r, RowDesc desc,
+                                           unsigned dst, int e0, int e1, int written) {
+  const int lane = threadIdx.x & 31;
+  int32_t* col = side == 0 ? p.g.out_col : p.g.in_col;
+  int32_t* w = side == 0 ? p.g.out_w : p.g.in_w;
+  for (int base = e0; base < e1; base += 32) {
+    const int e = base + lane;
+    const int32_t x = e < e1 ? col[desc.start + e] : kDead;
+    const bool live = x >= 0;
+    const unsigned ballot = __ballot_sync(0xffffffffu, live);
+    const int pos = written + __popc(ballot & ((1u << lane) - 1));
+    if (live) {
+      col[dst + pos] = x;
+      for (int j = 0; j < p.k; ++j)
+        w[j * p.g.arena_cap + dst + pos] = w[j * p.g.arena_cap + desc.start + e];
+      if (!p.g.allow_multi) {
+        const long long ie = index_find(p.g, side == 0 ? edge_key(r, x) : edge_key(x, r));
+        if (ie >= 0) *(side == 0 ? &p.g.eidx[ie].out : &p.g.eidx[ie].in) = dst + pos;
+        else set_error(&p.ctl->error, kErrInternal);
+      }
+    }
+    written += __popc(ballot);
+  }
+}
+
 // A warp takes the touched rows 32 at a time, each lane reading one row's relocation flag and
 // length; the warp then moves the flagged rows that hold slots one after another (lanes over the
 // row's slots).  Most relocated rows are empty (a vertex without edges has no slack: its first
 // edge relocates it, at R-MAT scale 22 about 70k rows per 100k-change batch), and they have
-// nothing to move, so they take no warp step.
+// nothing to move, so they take no warp step.  Rows longer than kMoveChunk follow, a chunk per warp.
 __device__ void ph_move(const ApplyParams& p, long long tid, long long threads) {
   UpdateCtl* c = p.ctl;
   const int lane = threadIdx.x & 31;
@@ -863,8 +942,10 @@ __device__ void ph_move(const ApplyParams& p, long long tid, long long threads) 
       const int side = mine < rows_out ? 0 : 1;
       const int s = side == 0 ? static_cast<int>(mine) : static_cast<int>(mine - rows_out);
       const int32_t r = (side == 0 ? p.rows_out : p.rows_in)[s];
-      if ((side == 0 ? p.reloc_out : p.reloc_in)[s] != 0 && r < c->n_old)
-        flagged = (side == 0 ? p.g.out_desc : p.g.in_desc)[r].len > 0;
+      if ((side == 0 ? p.reloc_out : p.reloc_in)[s] != 0 && r < c->n_old) {
+        const int len = (side == 0 ? p.g.out_desc : p.g.in_desc)[r].len;
+        flagged = len > 0 && len <= static_cast<int>(kMoveChunk);
+      }
     }
     unsigned todo = __ballot_sync(0xffffffffu, flagged);
     while (todo) {
@@ -874,29 +955,23 @@ __device__ void ph_move(const ApplyParams& p, long long tid, long long threads) 
       const int s = side == 0 ? static_cast<int>(i) : static_cast<int>(i - rows_out);
       const int32_t r = (side == 0 ? p.rows_out : p.rows_in)[s];
       const RowDesc desc = (side == 0 ? p.g.out_desc : p.g.in_desc)[r];
-      const unsigned dst = (side == 0 ? p.new_start_out : p.new_start_in)[s];
-      int32_t* col = side == 0 ? p.g.out_col : p.g.in_col;
-      int32_t* w = side == 0 ? p.g.out_w : p.g.in_w;
-      int written = 0;
-      for (int base = 0; base < desc.len; base += 32) {
-        const int e = base + lane;
-        const int32_t x = e < desc.len ? col[desc.start + e] : kDead;
-        const bool live = x >= 0;
-        const unsigned ballot = __ballot_sync(0xffffffffu, live);
-        const int pos = written + __popc(ballot & ((1u << lane) - 1));
-        if (live) {
-          col[dst + pos] = x;
-          for (int j = 0; j < p.k; ++j)
-            w[j * p.g.arena_cap + dst + pos] = w[j * p.g.arena_cap + desc.start + e];
-          if (!p.g.allow_multi) {
-            const long long ie = index_find(p.g, side == 0 ? edge_key(r, x) : edge_key(x, r));
-            if (ie >= 0) *(side == 0 ? &p.g.eidx[ie].out : &p.g.eidx[ie].in) = dst + pos;
-            else set_error(&c->error, kErrInternal);
-          }
-        }
-        written += __popc(ballot);
-      }
+      move_slots(p, side, r, desc, (side == 0 ? p.new_start_out : p.new_start_in)[s], 0, desc.len, 0);
     }
+  }
+  const int count = static_cast<int>(c->move_heavy >> 40);
+  const int chunks = static_cast<int>(c->move_heavy & ((1ULL << 40) - 1));
+  for (long long ch = warp; ch < chunks; ch += warps) {
+    const int2 at = find_move(p, count, static_cast<int>(ch));
+    const int side = at.x < rows_out ? 0 : 1;
+    const int s = side == 0 ? at.x : at.x - rows_out;
+    const int32_t r = (side == 0 ? p.rows_out : p.rows_in)[s];
+    const RowDesc desc = (side == 0 ? p.g.out_desc : p.g.in_desc)[r];
+    int before = 0;
+    for (int q = at.y + lane; q < ch; q += 32) before += __ldcg(&p.move_live[q]);
+    before = __reduce_add_sync(0xffffffffu, before);
+    const int e0 = static_cast<int>(ch - at.y) * static_cast<int>(kMoveChunk);
+    move_slots(p, side, r, desc, (side == 0 ? p.new_start_out : p.new_start_in)[s], e0,
+               min(desc.len, e0 + static_cast<int>(kMoveChunk)), before);
   }
 }
 
@@ -1380,7 +1455,12 @@ __global__ void __launch_bounds__(kBlock, 3) k_apply(ApplyParams p, ApplyLaunch 
   ph_mutate(p, red, tid, threads);
   if (!grid_sync(c, gen, arrivals, limit, &err) || err != 0) return;
   mark();
-  // H, I: relocated rows moved and new slots appended (disjoint slots)
+  // H, I: relocated rows moved and new slots appended (disjoint slots); long rows in chunks, whose
+  // live slots are counted first (every block reads the same count: written before F's barrier)
+  if (c->move_heavy != 0) {
+    ph_move_count(p, tid, threads);
+    if (!grid_sync(c, gen, arrivals, limit, &err) || err != 0) return;
+  }
   ph_move(p, tid, threads);
   ph_append(p, red, tid, threads);
   if (!grid_sync(c, gen, arrivals, limit, &err) || err != 0) return;
@@ -1405,7 +1485,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_apply(ApplyParams p, ApplyLaunch 
 // one block; `mark` >= 0 records the end of the previous step in apply_ns[mark].
 enum ApplyStep {
   kStepValidate, kStepPlan, kStepPairs, kStepMatch, kStepResolve, kStepRowOffsets,
-  kStepFillSegments, kStepSortSegments, kStepAlloc, kStepMutate, kStepMove, kStepAppend,
+  kStepFillSegments, kStepSortSegments, kStepAlloc, kStepMutate, kStepMoveCount, kStepMove, kStepAppend,
   kStepRows, kStepFinalize
 };
 
@@ -1447,6 +1527,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_apply_step(ApplyParams p, ApplyLa
       if (tid == 0) c->committing = 1;
       ph_mutate(p, red, tid, threads);
       break;
+    case kStepMoveCount: ph_move_count(p, tid, threads); break;
     case kStepMove: ph_move(p, tid, threads); break;  // H and I touch disjoint slots
     case kStepAppend: ph_append(p, red, tid, threads); break;
     case kStepRows:
@@ -1533,6 +1614,8 @@ ApplyParams make_params(Context& ctx, Graph& g, const StagedBatch& b, int object
   p.new_cap_in = ws.row_new_cap_in.ptr;
   p.live_out = ws.row_live_out.ptr;
   p.live_in = ws.row_live_in.ptr;
+  p.move_list = reinterpret_cast<int2*>(ws.move_list.ptr);
+  p.move_live = ws.move_live.ptr;
   p.col_sum_delta = ws.col_sum_delta.ptr;
   p.col_removed_at_max = ws.col_removed_at_max.ptr;
   p.col_written_max = ws.col_written_max.ptr;
@@ -2215,6 +2298,13 @@ void apply_launch(Context& ctx, Graph& g, const StagedBatch& b, int objective, l
   // every allocation first: a failed one leaves the graph as it was
   ws.reserve_vertices(g.n_cap, s);
   ws.reserve_batch(ops, g.k, s);
+  {
+    // rows longer than a chunk, at most arena_cap / kMoveChunk on each side; their chunks, at most
+    // twice as many
+    const size_t rows = 2 * (static_cast<size_t>(g.arena_cap) / kMoveChunk + 1);
+    ws.move_list.reserve(2 * rows);  // int2 entries
+    ws.move_live.reserve(2 * rows);
+  }
   if (!g.props.sorted) {
     const size_t cap = static_cast<size_t>(ws.pairs_sized);
     ws.row_seg_offsets.reserve(cap);
@@ -2257,8 +2347,8 @@ void apply_launch(Context& ctx, Graph& g, const StagedBatch& b, int objective, l
     int mark = 0;
     auto step = [&](int which, int grid) {
       // the plan and the pairs, and the moves and the appends, are one step each in the fused
-      // kernel: the second of each pair records no mark
-      const bool second = which == kStepPairs || which == kStepAppend;
+      // kernel: the later launches of each record no mark
+      const bool second = which == kStepPairs || which == kStepMove || which == kStepAppend;
       k_apply_step<<<grid, kBlock, 0, s>>>(p, L, which, second ? -1 : mark);
       if (!second) ++mark;
       ++ctx.launches;
@@ -2276,6 +2366,7 @@ void apply_launch(Context& ctx, Graph& g, const StagedBatch& b, int objective, l
     }
     step(kStepAlloc, blocks);
     step(kStepMutate, blocks);
+    step(kStepMoveCount, blocks);
     step(kStepMove, blocks);
     step(kStepAppend, blocks);
     step(kStepRows, blocks);

@@ -126,6 +126,7 @@ struct UpdateCtl {
   int chunks_out, chunks_in;
   int relocated_out, relocated_in;
   int pad1;
+  u64 move_heavy;       // (rows << 40 | chunks) of the long relocated rows
   u64 top_out, top_in;  // tentative arena tops
   u64 seg_top;          // append-order rows: segments reserved so far
   int committing;       // the applier passed its allocation step: the graph is being changed
@@ -218,6 +219,7 @@ struct Workspace {
   DevBuf<unsigned> row_append_at_out, row_append_at_in;  // first append slot of each touched row
   DevBuf<int> row_new_cap_out, row_new_cap_in, row_live_out, row_live_in;
   DevBuf<int> row_seg_offsets, row_seg;  // append order: appended pairs per row
+  DevBuf<int> move_list, move_live;      // long relocated rows: (row, first chunk); live slots
   DevBuf<long long> col_ins_max, col_sum_delta, col_removed_at_max, col_written_max,
       col_written_at_max;
   // batch staging

@@ -65,9 +65,12 @@ struct ApplyParams {
   int objective;
   dyngb200_props props;
   long long delta_opt;
-  // pair table
-  u64* key;
+  // pair table (hashed), and the pairs' fields by their place in the list: step C groups the
+  // operations in the table, step D copies each pair's entry out of it, and from there on every
+  // step reads and writes the fields by coalesced passes over the list
+  PairSlot* table;
   int mask;
+  u64* key;
   int* d;
   int* t;
   int* first;
@@ -81,7 +84,9 @@ struct ApplyParams {
   int* in_rank;
   int* out_count;  // matches in the out row (multi-edge graphs)
   int* in_count;
-  int* list;
+  int* row_out;  // the touched-row slots of u and v (pairs that change a row)
+  int* row_in;
+  int* list;  // the pairs' table slots
   unsigned char* inc;
   // touched rows
   int* touch_out_stamp;
@@ -134,15 +139,36 @@ enum : int {
   kPairUseFirst = 32,    // the first insertion's weights (ignore semantics), else the last's
 };
 
+// The place in the list of a pair of the batch (-1: not in it).
 __device__ __forceinline__ int find_pair(const ApplyParams& p, u64 k) {
   unsigned h = static_cast<unsigned>(mix64(k)) & static_cast<unsigned>(p.mask);
   for (int probe = 0; probe <= p.mask; ++probe) {
-    const u64 cur = p.key[h];
-    if (cur == k) return static_cast<int>(h);
+    const u64 cur = p.table[h].key;
+    if (cur == k) return p.table[h].id;
     if (cur == kEmptyKey) return -1;
     h = (h + 1) & static_cast<unsigned>(p.mask);
   }
   return -1;
+}
+
+// Pair i's entry of the table into its fields.
+__device__ __forceinline__ PairSlot load_pair(const ApplyParams& p, long long i, bool write) {
+  PairSlot* at = &p.table[p.list[i]];
+  union {
+    int4 raw[2];
+    PairSlot s;
+  } e;
+  e.raw[0] = __ldcg(reinterpret_cast<const int4*>(at));
+  e.raw[1] = __ldcg(reinterpret_cast<const int4*>(at) + 1);
+  if (write) {
+    p.key[i] = e.s.key;
+    p.d[i] = e.s.d;
+    p.t[i] = e.s.t;
+    p.first[i] = e.s.first;
+    p.last[i] = e.s.last;
+    if (p.objective < 0) at->id = static_cast<int>(i);  // graph::apply's classification looks pairs up
+  }
+  return e.s;
 }
 
 // ---- A: Step 0 checks, vertex growth, largest insertion weight --------------------------------
@@ -240,20 +266,12 @@ __device__ void ph_validate(const ApplyParams& p, BlockRed& R, long long tid, lo
 __device__ void ph_clear(const ApplyParams& p, long long tid, long long threads) {
   const long long cap = static_cast<long long>(p.mask) + 1;
   const int k = p.k > 0 ? p.k : 1;
-  // every field a new pair starts from, written here by coalesced passes over the table rather
-  // than by the thread that inserts the pair (one scattered 32-byte sector per field and pair)
+  // what a new pair starts from, written here by a coalesced pass over the table rather than by
+  // the thread that inserts the pair
+  const int4 lo = make_int4(-1, -1, 0, 0), hi = make_int4(0x7f7f7f7f, -1, -1, 0);
   for (long long i = tid; i < cap; i += threads) {
-    p.key[i] = ~0ULL;
-    p.d[i] = 0;
-    p.t[i] = 0;
-    p.first[i] = 0x7f7f7f7f;
-    p.last[i] = -1;
-    p.out_pos[i] = -1;
-    p.in_pos[i] = -1;
-    p.out_pos2[i] = -1;
-    p.in_pos2[i] = -1;
-    p.out_count[i] = 0;
-    p.in_count[i] = 0;
+    reinterpret_cast<int4*>(p.table)[2 * i] = lo;
+    reinterpret_cast<int4*>(p.table)[2 * i + 1] = hi;
     if (i < k) {
       p.col_sum_delta[i] = 0;
       p.col_removed_at_max[i] = 0;
@@ -336,7 +354,7 @@ __device__ void add_op(PairStage& st, const ApplyParams& p, int32_t u, int32_t v
   unsigned h = static_cast<unsigned>(mix64(k)) & static_cast<unsigned>(p.mask);
   int slot = -1;
   for (int probe = 0; probe <= p.mask; ++probe) {
-    const u64 prev = atomicCAS(&p.key[h], kEmptyKey, k);
+    const u64 prev = atomicCAS(&p.table[h].key, kEmptyKey, k);
     if (prev == kEmptyKey) {
       slot = static_cast<int>(h);  // its fields were set by the clear step
       stage_put(st, p, 0, slot);
@@ -355,11 +373,11 @@ __device__ void add_op(PairStage& st, const ApplyParams& p, int32_t u, int32_t v
     return;
   }
   if (kind == 0) {
-    atomicAdd(&p.d[slot], 1);
+    atomicAdd(&p.table[slot].d, 1);
   } else {
-    atomicAdd(&p.t[slot], 1);
-    atomicMin(&p.first[slot], index);
-    atomicMax(&p.last[slot], index);
+    atomicAdd(&p.table[slot].t, 1);
+    atomicMin(&p.table[slot].first, index);
+    atomicMax(&p.table[slot].last, index);
   }
 }
 
@@ -422,16 +440,14 @@ __device__ void ph_match(const ApplyParams& p, long long tid, long long threads)
   UpdateCtl* c = p.ctl;
   const int pairs = c->pairs;
   for (long long i = tid; i < pairs; i += threads) {
-    const int slot = p.list[i];
-    EdgeSlot at;
-    const long long e = index_find(p.g, p.key[slot], &at);
-    if (e >= 0) {
-      p.out_pos[slot] = static_cast<int>(at.out);
-      p.in_pos[slot] = static_cast<int>(at.in);
-      p.out_count[slot] = 1;
-      p.in_count[slot] = 1;
-    }
-    p.in_pos2[slot] = static_cast<int>(e);  // index slot of the pair (or -1)
+    const PairSlot pair = load_pair(p, i, true);
+    EdgeSlot at{0, ~0u, ~0u};
+    const long long e = index_find(p.g, pair.key, &at);
+    p.out_pos[i] = static_cast<int>(at.out);
+    p.in_pos[i] = static_cast<int>(at.in);
+    p.out_count[i] = e >= 0 ? 1 : 0;
+    p.in_count[i] = e >= 0 ? 1 : 0;
+    p.in_pos2[i] = static_cast<int>(e);  // index slot of the pair (or -1)
   }
 }
 
@@ -443,14 +459,22 @@ __device__ void ph_scan_multi(const ApplyParams& p, long long tid, long long thr
   const int pairs = c->pairs;
   const int lane = threadIdx.x & 31;
   for (long long i = tid >> 5; i < pairs; i += threads >> 5) {
-    const int slot = p.list[i];
-    const u64 key = p.key[slot];
+    const int slot = static_cast<int>(i);
+    const PairSlot pair = load_pair(p, i, lane == 0);
+    const u64 key = pair.key;
     const int32_t u = static_cast<int32_t>(key >> 32), v = static_cast<int32_t>(key & 0xffffffffu);
-    const int d = p.d[slot];
+    const int d = pair.d;
     for (int side = 0; side < 2; ++side) {
       const int32_t r = side == 0 ? u : v;
       const int32_t want = side == 0 ? v : u;
-      if (r >= c->n_old) continue;
+      if (r >= c->n_old) {  // a vertex the batch brings: no match
+        if (lane == 0) {
+          (side == 0 ? p.out_count : p.in_count)[slot] = 0;
+          (side == 0 ? p.out_pos : p.in_pos)[slot] = -1;
+          (side == 0 ? p.out_pos2 : p.in_pos2)[slot] = -1;
+        }
+        continue;
+      }
       const RowDesc desc = (side == 0 ? p.g.out_desc : p.g.in_desc)[r];
       const int32_t* col = (side == 0 ? p.g.out_col : p.g.in_col) + desc.start;
       // first match, and match number d (the first survivor of the deletions); absolute slots
@@ -492,7 +516,7 @@ __device__ void ph_resolve(const ApplyParams& p, BlockRed& R, long long tid, lon
   const int policy = p.props.on_existing_insert;
   long long acc[5] = {0, 0, 0, 0, 0};
   for (long long i = tid; i < pairs; i += threads) {
-    const int slot = p.list[i];
+    const int slot = static_cast<int>(i);
     const u64 key = p.key[slot];
     const int32_t u = static_cast<int32_t>(key >> 32), v = static_cast<int32_t>(key & 0xffffffffu);
     const int d = p.d[slot];
@@ -572,6 +596,8 @@ __device__ void ph_resolve(const ApplyParams& p, BlockRed& R, long long tid, lon
     if (tomb || app) {
       const int so = p.row_slot_out[u];
       const int si = p.row_slot_in[v];
+      p.row_out[slot] = so;
+      p.row_in[slot] = si;
       if (tomb) {
         atomicAdd(&p.dels_out[so], tomb);
         atomicAdd(&p.dels_in[si], tomb);
@@ -767,7 +793,7 @@ __device__ void ph_mutate(const ApplyParams& p, BlockRed& R, long long tid, long
   const long long first_i = multi ? tid >> 5 : tid;
   const long long step = multi ? threads >> 5 : threads;
   for (long long i = first_i; i < pairs; i += step) {
-    const int slot = p.list[i];
+    const int slot = static_cast<int>(i);
     const u64 key = p.key[slot];
     const int32_t u = static_cast<int32_t>(key >> 32), v = static_cast<int32_t>(key & 0xffffffffu);
     const int d = p.d[slot];
@@ -983,7 +1009,7 @@ __device__ void ph_append(const ApplyParams& p, BlockRed& R, long long tid, long
   acc_init(acc);
   long long idx_new = 0, idx_reused = 0;
   for (long long i = tid; i < pairs; i += threads) {
-    const int slot = p.list[i];
+    const int slot = static_cast<int>(i);
     const int flags = p.flags[slot];
     if (!(flags & kPairAppend)) continue;
     const u64 key = p.key[slot];
@@ -992,7 +1018,7 @@ __device__ void ph_append(const ApplyParams& p, BlockRed& R, long long tid, long
     // both sides' loads first (they are independent), then the stores; the row's first append
     // slot (after its live slots if it moved, after its old length if not) was set by the alloc
     // step, so one scattered row field is read per side
-    const int s0 = p.row_slot_out[u], s1 = p.row_slot_in[v];
+    const int s0 = p.row_out[slot], s1 = p.row_in[slot];
     const int rk0 = p.out_rank[slot], rk1 = p.in_rank[slot];
     const unsigned placed[2] = {p.append_at_out[s0] + rk0, p.append_at_in[s1] + rk1};
     p.g.out_col[placed[0]] = v;
@@ -1082,7 +1108,7 @@ __device__ void ph_count_written_max(const ApplyParams& p, BlockRed& R, long lon
   ColumnAcc acc;
   acc_init(acc);
   for (long long i = tid; i < pairs; i += threads) {
-    const int slot = p.list[i];
+    const int slot = static_cast<int>(i);
     const int flags = p.flags[slot];
     if (!(flags & (kPairAppend | kPairUpsert))) continue;
     const int ins_index = (flags & kPairUseFirst) ? p.first[slot] : p.last[slot];
@@ -1207,10 +1233,9 @@ __device__ void ph_fill_segments(const ApplyParams& p, const int* offsets, int* 
   UpdateCtl* c = p.ctl;
   const int pairs = c->pairs;
   for (long long i = tid; i < pairs; i += threads) {
-    const int slot = p.list[i];
+    const int slot = static_cast<int>(i);
     if (!(p.flags[slot] & kPairAppend)) continue;
-    const int32_t u = static_cast<int32_t>(p.key[slot] >> 32);
-    seg[offsets[p.row_slot_out[u]] + p.out_rank[slot]] = slot;
+    seg[offsets[p.row_out[slot]] + p.out_rank[slot]] = slot;
   }
 }
 
@@ -1577,6 +1602,7 @@ ApplyParams make_params(Context& ctx, Graph& g, const StagedBatch& b, int object
   p.objective = objective;
   p.props = g.props;
   p.delta_opt = delta_opt;
+  p.table = ws.pair_table.ptr;
   p.key = ws.pair_key.ptr;
   p.mask = static_cast<int>(ws.pairs_active - 1);
   p.d = ws.pair_d.ptr;
@@ -1592,6 +1618,8 @@ ApplyParams make_params(Context& ctx, Graph& g, const StagedBatch& b, int object
   p.in_rank = ws.pair_in_rank.ptr;
   p.out_count = ws.pair_out_row.ptr;
   p.in_count = ws.pair_in_row.ptr;
+  p.row_out = ws.pair_row_out.ptr;
+  p.row_in = ws.pair_row_in.ptr;
   p.list = ws.pair_list.ptr;
   p.inc = ws.pair_inc.ptr;
   p.touch_out_stamp = ws.touch_out_stamp.ptr;
@@ -1669,32 +1697,38 @@ void Workspace::reserve_batch(long long ops, int k, cudaStream_t s) {
   if (cap > pairs_sized) {
     const size_t c = static_cast<size_t>(cap);
     pairs_sized = 0;  // unsized until every table is back (see reserve_vertices)
+    pair_table.release();
+    pair_table.reserve(c, s);
+    // the lists hold at most one pair, and one touched row per side, per directed operation: half
+    // the table
+    const size_t half = c / 2;
     pair_key.release();
-    pair_key.reserve(c, s);
+    pair_key.reserve(half, s);
     for (DevBuf<int>* b : {&pair_d, &pair_t, &pair_first, &pair_last, &pair_out_pos, &pair_in_pos,
                            &pair_out_pos2, &pair_in_pos2, &pair_flags, &pair_out_row,
-                           &pair_in_row, &pair_out_rank, &pair_in_rank, &pair_list}) {
+                           &pair_in_row, &pair_out_rank, &pair_in_rank, &pair_list, &pair_row_out,
+                           &pair_row_in}) {
       b->release();
-      b->reserve(c, s);
+      b->reserve(half, s);
     }
     for (DevBuf<int>* b : {&rows_out, &rows_in, &row_dels_out, &row_dels_in, &row_apps_out,
                            &row_apps_in, &row_reloc_out, &row_reloc_in, &row_new_cap_out,
                            &row_new_cap_in, &row_live_out, &row_live_in}) {
       b->release();
-      b->reserve(c, s);
+      b->reserve(half, s);
     }
     row_new_start_out.release();
-    row_new_start_out.reserve(c, s);
+    row_new_start_out.reserve(half, s);
     row_new_start_in.release();
-    row_new_start_in.reserve(c, s);
+    row_new_start_in.reserve(half, s);
     row_append_at_out.release();
-    row_append_at_out.reserve(c, s);
+    row_append_at_out.reserve(half, s);
     row_append_at_in.release();
-    row_append_at_in.reserve(c, s);
+    row_append_at_in.reserve(half, s);
     pairs_sized = cap;
   }
   pairs_active = cap;
-  const size_t inc = static_cast<size_t>(pairs_sized) * static_cast<size_t>(k > 0 ? k : 1);
+  const size_t inc = static_cast<size_t>(pairs_sized / 2) * static_cast<size_t>(k > 0 ? k : 1);
   pair_inc.reserve(inc, s);
   for (DevBuf<long long>* b : {&col_ins_max, &col_sum_delta, &col_removed_at_max,
                                &col_written_max, &col_written_at_max}) {

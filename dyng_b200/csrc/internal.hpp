@@ -205,12 +205,23 @@ constexpr int kClaimBlockBits = 10;
 static_assert((1 << kClaimBlockBits) >= kPjMaxBlocks, "a claim names the block");
 constexpr int kMaxGeneration = (1 << (31 - kClaimBlockBits)) - 1;
 
+// A (u, v) pair of a batch in the applier's hash table: one 32-byte sector.  `d` deletions, `t`
+// insertions, the first and last insertion; `id`, the pair's place in the list (graph::apply).
+struct alignas(32) PairSlot {
+  u64 key;
+  int d, t;
+  int first, last;
+  int id, pad;
+};
+
 // Scratch memory of a context, sized on demand and reused (the reference's workspace pool).
 struct Workspace {
   // applier
+  DevBuf<PairSlot> pair_table;
   DevBuf<u64> pair_key;
   DevBuf<int> pair_d, pair_t, pair_first, pair_last, pair_out_pos, pair_in_pos, pair_out_pos2,
-      pair_in_pos2, pair_flags, pair_out_row, pair_in_row, pair_out_rank, pair_in_rank, pair_list;
+      pair_in_pos2, pair_flags, pair_out_row, pair_in_row, pair_out_rank, pair_in_rank, pair_list,
+      pair_row_out, pair_row_in;
   DevBuf<unsigned char> pair_inc;  // pairs x k weight-increase flags
   DevBuf<int> touch_out_stamp, touch_in_stamp, row_slot_out, row_slot_in;
   DevBuf<int> rows_out, rows_in;  // touched row ids

@@ -138,7 +138,7 @@ __global__ void k_op_roots(SsspParams p, int gen_inv, int* level, int walk, OpCo
   long long inval = 0;
   int changed = 0;
   for (long long i = op_tid(); i < pairs; i += op_threads()) {
-    const int slot = p.pair_list[i];
+    const int slot = static_cast<int>(i);
     const int f = p.pair_flags[slot];
     const bool increased = p.use_inc ? p.inc[static_cast<long long>(slot) * p.k + p.objective] != 0
                                      : (f & kPairIncreased) != 0;
@@ -225,7 +225,7 @@ __global__ void k_op_heads(SsspParams p, int bits, u64 maxd, int gen_inv, int ge
   const Packing pk = packing_of(bits);
   const int pairs = p.ctl->pairs;
   for (long long i = op_tid(); i < pairs; i += op_threads()) {
-    const int slot = p.pair_list[i];
+    const int slot = static_cast<int>(i);
     const int f = p.pair_flags[slot];
     if (!(f & kPairHead)) continue;
     const u64 key = p.pair_key[slot];

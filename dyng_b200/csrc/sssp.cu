@@ -1018,7 +1018,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
     int changed = 0;
     for (long long i = tid; i < pairs; i += threads) {
       ++pair_visits;
-      const int slot = p.pair_list[i];
+      const int slot = static_cast<int>(i);
       const int f = p.pair_flags[slot];
       const bool increased = p.use_inc ? p.inc[static_cast<long long>(slot) * p.k + p.objective] != 0
                                        : (f & kPairIncreased) != 0;
@@ -1283,7 +1283,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
     if (tid == 0) c->phase_ns[3] = c->phase_ns[2];
     for (long long i = tid; i < pairs; i += threads) {
       ++pair_visits;
-      const int slot = p.pair_list[i];
+      const int slot = static_cast<int>(i);
       const int f = p.pair_flags[slot];
       if (!(f & kPairHead)) continue;
       const u64 key = p.pair_key[slot];
@@ -1760,7 +1760,6 @@ static void enqueue_attempt(PendingUpdate& u) {
   p.tree_n = t.n;
   p.tree_bits = t.packed_bits;
   p.pair_key = ws.pair_key.ptr;
-  p.pair_list = ws.pair_list.ptr;
   p.pair_flags = ws.pair_flags.ptr;
   p.pair_first = ws.pair_first.ptr;
   p.pair_last = ws.pair_last.ptr;
@@ -2037,7 +2036,6 @@ static void sssp_rerun(Context& ctx, Graph& g, Tree& t, const UpdateCtl& applied
   p.tree_n = t.n;
   p.tree_bits = t.packed_bits;
   p.pair_key = ws.pair_key.ptr;
-  p.pair_list = ws.pair_list.ptr;
   p.pair_flags = ws.pair_flags.ptr;
   p.pair_first = ws.pair_first.ptr;
   p.pair_last = ws.pair_last.ptr;

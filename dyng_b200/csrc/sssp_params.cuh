@@ -20,9 +20,8 @@ struct SsspParams {
   int walk;              // invalidation by a subtree walk instead of pointer jumping
   int tree_trusted;      // computed or validated: no parent cycle possible
   int offer_heads;       // canonical tree: insertion heads take the inserted edge's offer
-  // pairs of the applier (update only) and the batch weights
+  // pairs of the applier by their place in its list (update only) and the batch weights
   const u64* pair_key;
-  const int* pair_list;
   const int* pair_flags;
   const int* pair_first;
   const int* pair_last;

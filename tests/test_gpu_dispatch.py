@@ -1,0 +1,210 @@
+"""The branches that the update's kernels choose by size, each at the sizes where it can go wrong,
+against the oracle bit for bit:
+
+  - near-far steps that a block continues by itself: short frontiers of light rows, the hand-over
+    back to the grid, a chain longer than the claims' generations last;
+  - threshold raises that find nothing below the new threshold and skip to the next distance;
+  - relocated rows around the length above which a row moves in chunks;
+  - host batches around the size that comes over with the control block;
+  - the subtree walk that an update without a schedule tries when few tree edges changed.
+"""
+import numpy as np
+import pytest
+
+import dyng_b200 as D
+from oracle import oracle as O
+from tests.helpers import random_batch
+
+pytestmark = pytest.mark.gpu
+
+MOVE_CHUNK = 512          # slots of a row that move as one piece
+STAGED_VALUES = 64 * 1024 // 4  # values of a host batch that come over with the control block
+
+
+def _both(n, src, dst, w, props=None, oprops=None):
+    g = D.Graph.from_edges(src, dst, w, n, props)
+    og = O.Graph.from_edges(n, src, dst, w, 1, oprops)
+    t = D.sssp.compute(g, 0)
+    ot, _ = O.compute(og, 0, rule=1)
+    _same(t, ot, "compute")
+    return g, og, t, ot
+
+
+def _same(t, ot, label):
+    np.testing.assert_array_equal(t.distances, ot.distances, err_msg=label)
+    np.testing.assert_array_equal(t.parents, ot.parents, err_msg=label)
+
+
+def _update(g, og, t, ot, b, label, schedule=None):
+    st = D.sssp.update(g, D.EdgeBatch.from_arrays(b["ins_src"], b["ins_dst"], b["ins_w"],
+                                                  b["del_src"], b["del_dst"]), t, schedule)
+    ost, osm = O.update(og, O.Batch(b["ins_src"], b["ins_dst"], b["ins_w"], b["del_src"],
+                                    b["del_dst"]), ot)
+    _same(t, ot, label)
+    assert (st.invalidated, st.affected) == (ost["invalidated"], ost["affected"]), label
+    assert st.batch.inserted_edges == osm["inserted_edges"], label
+    assert st.batch.deleted_edges == osm["deleted_edges"], label
+    return st
+
+
+def _csr_same(g, og):
+    csr, want = g.to_csr(), og.to_csr()
+    np.testing.assert_array_equal(csr.row_ptr, want["row_ptr"])
+    np.testing.assert_array_equal(csr.col_ind, want["col"])
+    np.testing.assert_array_equal(csr.weights, want["w"])
+
+
+def _i32(*a):
+    return [np.asarray(x, np.int32) for x in a]
+
+
+def _grid(side, rng, w_max):
+    v = np.arange(side * side)
+    x, y = v % side, v // side
+    right, down = v[x + 1 < side], v[y + 1 < side]
+    src = np.concatenate([right, right + 1, down, down + side])
+    dst = np.concatenate([right + 1, right, down + side, down])
+    return side * side, *_i32(src, dst, rng.integers(1, w_max, src.size, endpoint=True))
+
+
+@pytest.mark.parametrize("side,delta", [(3, 0), (33, 1), (90, 0), (200, 0), (200, 1 << 40)])
+@pytest.mark.parametrize("small", [0, -1, 1, 100000])
+def test_short_frontiers_of_light_rows(side, delta, small):
+    rng = np.random.default_rng(side)
+    n, src, dst, w = _grid(side, rng, 50)
+    g, og, t, ot = _both(n, src, dst, w)
+    for step in range(3):
+        b = random_batch(rng, n, src, dst, max(4, n // 20), tree_parents=ot.parents)
+        _update(g, og, t, ot, b, f"step {step}", D.sssp.Schedule(delta=delta, small_frontier=small))
+
+
+def test_repeated_updates_of_one_grid_keep_the_same_tree():
+    # the same batch and its inverse again and again: a lost or doubled list entry anywhere shows
+    # as another tree sooner or later
+    rng = np.random.default_rng(8)
+    n, src, dst, w = _grid(160, rng, 40)
+    g, og, t, ot = _both(n, src, dst, w)
+    pick = rng.choice(src.size, 900, replace=False)
+    there = dict(ins_src=src[:0], ins_dst=dst[:0], ins_w=w[:0], del_src=src[pick], del_dst=dst[pick])
+    back = dict(ins_src=src[pick], ins_dst=dst[pick], ins_w=w[pick], del_src=src[:0], del_dst=dst[:0])
+    _update(g, og, t, ot, there, "there")
+    want = ot.distances.copy(), ot.parents.copy()
+    _update(g, og, t, ot, back, "back")
+    home = ot.distances.copy(), ot.parents.copy()
+    for i in range(400):
+        for b, (d, p) in ((there, want), (back, home)):
+            D.sssp.update(g, D.EdgeBatch.from_arrays(*b.values()), t)
+            np.testing.assert_array_equal(t.distances, d, err_msg=str(i))
+            np.testing.assert_array_equal(t.parents, p, err_msg=str(i))
+
+
+def test_a_chain_longer_than_the_claims_generations():
+    # 2^21 + 4096 dependent rounds in one call; then an update whose claims start over
+    n = (1 << 21) + 4096
+    src = np.arange(n - 1, dtype=np.int32)
+    w = np.ones(n - 1, np.int32)
+    g = D.Graph.from_edges(src, src + 1, w, n)
+    t, st = D.sssp.compute(g, 0, stats=True)
+    assert st.iterations >= n - 1
+    np.testing.assert_array_equal(t.distances, np.arange(n))
+    cut = n - 1000
+    D.sssp.update(g, D.EdgeBatch(insert=([0], [cut], [5]), delete=([cut - 1], [cut])), t)
+    want = np.arange(n)
+    want[cut:] = 5 + np.arange(n - cut)
+    np.testing.assert_array_equal(t.distances, want)
+
+
+@pytest.mark.parametrize("gap", [1, 7, 1 << 20, 2**31 - 1])
+def test_threshold_raises_over_gaps(gap):
+    # chains whose edges weigh 1 or `gap`: with width 1 most raises find nothing
+    rng = np.random.default_rng(3)
+    n = 300
+    src = np.concatenate([np.arange(n - 1), rng.integers(0, n, 60)])
+    dst = np.concatenate([np.arange(1, n), rng.integers(0, n, 60)])
+    w = np.where(rng.random(src.size) < 0.1, gap, 1)
+    src, dst, w = _i32(src, dst, w)
+    g, og, t, ot = _both(n, src, dst, w)
+    for step in range(3):
+        b = random_batch(rng, n, src, dst, 20, tree_parents=ot.parents)
+        _update(g, og, t, ot, b, f"step {step}", D.sssp.Schedule(delta=1))
+
+
+@pytest.mark.parametrize("kind", ["sorted", "append", "undirected", "multi"])
+@pytest.mark.parametrize("length", [1, MOVE_CHUNK - 1, MOVE_CHUNK, MOVE_CHUNK + 1,
+                                    2 * MOVE_CHUNK + 3, 5 * MOVE_CHUNK])
+def test_relocated_rows_around_the_chunk_length(kind, length):
+    # two hubs of `length` out-edges (and one of `length` in-edges) lose a third of their edges,
+    # which leaves tombstones in every chunk, and take enough new ones to move
+    rng = np.random.default_rng(length)
+    n = 6 * MOVE_CHUNK + 64
+    props = dict(sorted=kind in ("sorted", "undirected"), allow_multi=kind == "multi",
+                 directed=kind != "undirected")
+    far = 10 + rng.permutation(n - 10)[:length]
+    src = np.concatenate([np.zeros(length), np.ones(length), far])
+    dst = np.concatenate([far, far, np.full(length, 2)])
+    src, dst = _i32(np.append(src, [0, 0]), np.append(dst, [1, 2]))
+    w = rng.integers(1, 100, src.size).astype(np.int32)
+    g, og, t, ot = _both(n, src, dst, w, D.GraphProperties(**props), O.default_props(
+        directed=int(props["directed"]), sorted=int(props["sorted"]),
+        allow_multi=int(props["allow_multi"])))
+    gone = rng.random(src.size) < 1 / 3
+    extra = 10 + rng.permutation(n - 10)[:length // 2 + 8]
+    ins_src = np.concatenate([np.zeros(extra.size), np.ones(extra.size), extra])
+    ins_dst = np.concatenate([extra, extra, np.full(extra.size, 2)])
+    b = dict(zip(("ins_src", "ins_dst", "ins_w", "del_src", "del_dst"),
+                 _i32(ins_src, ins_dst, rng.integers(1, 100, ins_src.size), src[gone], dst[gone])))
+    _update(g, og, t, ot, b, "move")
+    _csr_same(g, og)
+    # the moved edges are found again (the edge index followed them)
+    again = dict(ins_src=src[:0], ins_dst=dst[:0], ins_w=w[:0], del_src=src[~gone], del_dst=dst[~gone])
+    _update(g, og, t, ot, again, "delete the moved edges")
+    _csr_same(g, og)
+
+
+@pytest.mark.parametrize("values", [2, STAGED_VALUES - 1, STAGED_VALUES, STAGED_VALUES + 1])
+def test_host_batches_around_the_staged_size(values):
+    # an insertion is three values of a host batch, a deletion two
+    rng = np.random.default_rng(values)
+    n = 4000
+    src, dst = rng.integers(0, n, (2, 6 * n)).astype(np.int32)
+    w = rng.integers(1, 100, src.size).astype(np.int32)
+    g, og, t, ot = _both(n, src, dst, w)
+    deletions = next(d for d in range(3) if (values - 2 * d) % 3 == 0)
+    inserts = (values - 2 * deletions) // 3
+    for step in range(2):
+        pick = rng.integers(0, src.size, deletions)
+        i, j = rng.integers(0, n, (2, inserts)).astype(np.int32)
+        b = dict(ins_src=i, ins_dst=j, ins_w=rng.integers(1, 100, inserts).astype(np.int32),
+                 del_src=src[pick], del_dst=dst[pick])
+        _update(g, og, t, ot, b, f"step {step}")
+    _csr_same(g, og)
+
+
+@pytest.mark.parametrize("roots", [1, 31, 32, 33, 200])
+@pytest.mark.parametrize("depth", [1, 7, 60])
+def test_few_changed_tree_edges(roots, depth):
+    # a shallow dense part (six edges per vertex) with chains of `depth` below it: deleting the
+    # chains' first edges invalidates them; the walk reaches them or leaves the rest to the rounds
+    rng = np.random.default_rng(100 * roots + depth)
+    core = 3000
+    chains = 220
+    n = core + chains * depth
+    src = [rng.integers(0, core, 8 * n)]
+    dst = [rng.integers(0, core, 8 * n)]
+    w = [rng.integers(1, 50, 8 * n)]
+    heads = rng.choice(core, chains, replace=False)
+    first = core + np.arange(chains) * depth
+    src.append(heads), dst.append(first), w.append(np.ones(chains))
+    for k in range(1, depth):
+        src.append(first + k - 1), dst.append(first + k), w.append(np.ones(chains))
+    src, dst, w = _i32(np.concatenate(src), np.concatenate(dst), np.concatenate(w))
+    g, og, t, ot = _both(n, src, dst, w)
+    pick = rng.choice(chains, roots, replace=False)
+    empty = src[:0]
+    b = dict(ins_src=empty, ins_dst=empty, ins_w=empty,
+             del_src=heads[pick].astype(np.int32), del_dst=first[pick].astype(np.int32))
+    st = _update(g, og, t, ot, b, "cut")
+    assert st.invalidated == roots * depth
+    back = dict(ins_src=b["del_src"], ins_dst=b["del_dst"], ins_w=np.full(roots, 3, np.int32),
+                del_src=empty, del_dst=empty)
+    _update(g, og, t, ot, back, "mend")

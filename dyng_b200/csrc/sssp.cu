@@ -565,10 +565,15 @@ __device__ void expand(const SsspParams& p, Ctx& X, const int* light, int light_
   const RowDesc* descs = MODE == kPull ? p.g.in_desc : p.g.out_desc;
   // light: `per` consecutive vertices per warp, balanced so that every warp runs the same
   // number of rounds
+  // The classes start on different warps: the light rows on the first, the medium rows on the next
+  // free ones, the heavy chunks after those, so that a short frontier's rows of every class run side
+  // by side instead of one class after the other in the same warps.
+  long long taken = 0;  // warps with rows of the classes so far
   if (light_count > 0) {
     const long long rounds = (light_count + nwarps * 32 - 1) / (nwarps * 32);
     long long per = (light_count + rounds * nwarps - 1) / (rounds * nwarps);
     per = per < 1 ? 1 : (per > 32 ? 32 : per);
+    taken = min(nwarps, (light_count + per - 1) / per);
     for (long long base = gwarp * per; base < light_count; base += nwarps * per) {
       const long long i = base + lane;
       int owner = -1;
@@ -617,7 +622,8 @@ __device__ void expand(const SsspParams& p, Ctx& X, const int* light, int light_
       for (; i < end; ++i) medium_row(i);
     }
   } else {
-    for (long long i = gwarp; i < med_count; i += nwarps) medium_row(i);
+    const long long first = gwarp - taken;
+    for (long long i = first < 0 ? first + nwarps : first; i < med_count; i += nwarps) medium_row(i);
   }
   part_done(1);
   // heavy: chunks
@@ -650,7 +656,8 @@ __device__ void expand(const SsspParams& p, Ctx& X, const int* light, int light_
       for (long long c = static_cast<long long>(ch); c < end; ++c) heavy_chunk(c);
     }
   } else {
-    for (long long ch = gwarp; ch < chunks; ch += nwarps) heavy_chunk(ch);
+    const long long first = gwarp - (taken + med_count) % nwarps;
+    for (long long ch = first < 0 ? first + nwarps : first; ch < chunks; ch += nwarps) heavy_chunk(ch);
   }
   part_done(2);
   if (probe) {

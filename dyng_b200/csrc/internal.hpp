@@ -233,7 +233,11 @@ struct Workspace {
   DevBuf<int> move_list, move_live;      // long relocated rows: (row, first chunk); live slots
   DevBuf<long long> col_ins_max, col_sum_delta, col_removed_at_max, col_written_max,
       col_written_at_max;
-  // batch staging
+  // batch staging: a small host batch in one piece (page-locked copy, device copy, 16-byte words
+  // the next control-block upload brings over with it), larger ones array by array
+  HostBuf<int4> stage_host;
+  DevBuf<int4> stage_dev;
+  int stage_words = 0;
   DevBuf<int32_t> b_ins_src, b_ins_dst, b_ins_w, b_del_src, b_del_dst;
   // sssp
   DevBuf<int> stamp, touch_stamp, near_stamp, in_far, ancestor;
@@ -424,6 +428,9 @@ void scheduler_train(Context& ctx, Scheduler& s, const float* x, const int32_t* 
 struct InferArgs;
 void learned_infer_args(Context& ctx, Tree& t, const Scheduler* sch, InferArgs* out);
 
+// The pinned read-back area of a graph: the counters first, then the column statistics.
+constexpr size_t kCounterSlots = (sizeof(GraphCounters) + sizeof(ColumnStats) - 1) / sizeof(ColumnStats);
+
 // graph.cu
 void graph_build(Context& ctx, Graph& g, long long n, const int64_t* row_ptr, const int32_t* col,
                  const int32_t* w_objective_major, long long m);
@@ -453,7 +460,12 @@ void apply_launch(Context& ctx, Graph& g, const StagedBatch& b, int objective,
                   long long delta_opt, const dyngb200_schedule* sched, Tree* tree = nullptr,
                   const Scheduler* learned = nullptr, bool stepped = false);
 void schedule_into(const dyngb200_schedule& sched, UpdateCtl& init);
-StagedBatch stage_batch(Context& ctx, const dyngb200_batch& batch, int k);
+// `defer`: a small host batch may come over with the next upload_control instead of now.
+StagedBatch stage_batch(Context& ctx, const dyngb200_batch& batch, int k, bool defer);
+// The control block `init` (and a deferred batch) to the device; the control block, and with `g`
+// the graph's counters and column statistics, back into pinned memory.  One small kernel each.
+void upload_control(Context& ctx, const UpdateCtl& init);
+void read_back_control(Context& ctx, Graph* g);
 
 // sssp.cu
 void sssp_compute(Context& ctx, Graph& g, Tree& t, dyngb200_stats* st);

@@ -1675,10 +1675,9 @@ void sssp_compute(Context& ctx, Graph& g, Tree& t, dyngb200_stats* st) {
   init.minimum = kPackedInf;
   const dyngb200_schedule sched = ctx.schedule_set ? ctx.schedule : dyngb200_schedule{};
   schedule_into(sched, init);
-  *ws.host_ctl.ptr = init;
-  DYNGB200_CUDA(cudaMemcpyAsync(ws.ctl.ptr, ws.host_ctl.ptr, sizeof(UpdateCtl),
-                                cudaMemcpyHostToDevice, s));
   tree_reserve(ctx, t, g.n_cap);
+  ws.stage_words = 0;
+  upload_control(ctx, init);
   SsspParams p = base_params(ctx, g, t);
   p.from_scratch = 1;
   p.tree_bits = pk.bits;
@@ -1696,8 +1695,7 @@ void sssp_compute(Context& ctx, Graph& g, Tree& t, dyngb200_stats* st) {
     else launch(ctx, p, blocks);
   }
   DYNGB200_CUDA(cudaEventRecord(e1, s));
-  DYNGB200_CUDA(cudaMemcpyAsync(ws.host_ctl.ptr, ws.ctl.ptr, sizeof(UpdateCtl),
-                                cudaMemcpyDeviceToHost, s));
+  read_back_control(ctx, nullptr);
   DYNGB200_CUDA(cudaStreamSynchronize(s));
   float ms = 0;
   cudaEventElapsedTime(&ms, e0, e1);
@@ -1737,8 +1735,6 @@ void sssp_compute(Context& ctx, Graph& g, Tree& t, dyngb200_stats* st) {
 }
 
 // update(): the applier, then the persistent kernel, then one read-back of the control block.
-// The pinned read-back area of a graph: the counters first, then the column statistics.
-constexpr size_t kCounterSlots = (sizeof(GraphCounters) + sizeof(ColumnStats) - 1) / sizeof(ColumnStats);
 
 // One attempt of an update, queued on the context's stream: the applier, the persistent kernel,
 // and the read-back of the control block, counters and column statistics into pinned memory.
@@ -1780,13 +1776,7 @@ static void enqueue_attempt(PendingUpdate& u) {
   if (u.operators) run_operators(ctx, p);
   else launch(ctx, p, u.blocks);
   DYNGB200_CUDA(cudaEventRecord(u.e2, s));
-  DYNGB200_CUDA(cudaMemcpyAsync(ws.host_ctl.ptr, ws.ctl.ptr, sizeof(UpdateCtl),
-                                cudaMemcpyDeviceToHost, s));
-  DYNGB200_CUDA(cudaMemcpyAsync(g.pinned.ptr, g.counters.ptr, sizeof(GraphCounters),
-                                cudaMemcpyDeviceToHost, s));
-  DYNGB200_CUDA(cudaMemcpyAsync(g.pinned.ptr + kCounterSlots, g.columns.ptr,
-                                g.host_columns.size() * sizeof(ColumnStats),
-                                cudaMemcpyDeviceToHost, s));
+  read_back_control(ctx, &g);
   u.host_us[2] += us_since(h1);
 }
 
@@ -1810,7 +1800,7 @@ void sssp_update_begin(Context& ctx, Graph& g, Tree& t, const dyngb200_batch& ba
   u.operators = select_engine(ctx, t.opt.cuda_engine);
   if (g.host_columns[t.opt.objective].dirty) graph_rescan_columns(ctx, g);
   graph_index_reserve(ctx, g, batch.num_insertions * (g.props.directed ? 1 : 2));
-  u.b = stage_batch(ctx, batch, g.k);
+  u.b = stage_batch(ctx, batch, g.k, true);
   u.blocks = persistent_blocks(ctx, sched);
   for (cudaEvent_t& e : ctx.update_events)
     if (!e) DYNGB200_CUDA(cudaEventCreate(&e));
@@ -2030,13 +2020,11 @@ static void sssp_rerun(Context& ctx, Graph& g, Tree& t, const UpdateCtl& applied
   init.minimum = kPackedInf;
   const dyngb200_schedule sched{};
   schedule_into(sched, init);
-  *ws.host_ctl.ptr = init;
   tree_reserve(ctx, t, g.n_cap);
   cudaEvent_t e1, e2;
   DYNGB200_CUDA(cudaEventCreate(&e1));
   DYNGB200_CUDA(cudaEventCreate(&e2));
-  DYNGB200_CUDA(cudaMemcpyAsync(ws.ctl.ptr, ws.host_ctl.ptr, sizeof(UpdateCtl),
-                                cudaMemcpyHostToDevice, s));
+  upload_control(ctx, init);
   const int blocks = persistent_blocks(ctx, sched);
   SsspParams p = base_params(ctx, g, t);
   p.from_scratch = 0;
@@ -2059,8 +2047,7 @@ static void sssp_rerun(Context& ctx, Graph& g, Tree& t, const UpdateCtl& applied
   if (operators) run_operators(ctx, p);
   else launch(ctx, p, blocks);
   DYNGB200_CUDA(cudaEventRecord(e2, s));
-  DYNGB200_CUDA(cudaMemcpyAsync(ws.host_ctl.ptr, ws.ctl.ptr, sizeof(UpdateCtl),
-                                cudaMemcpyDeviceToHost, s));
+  read_back_control(ctx, nullptr);
   DYNGB200_CUDA(cudaStreamSynchronize(s));
   const UpdateCtl r = *ws.host_ctl.ptr;
   ws.generation = std::max(ws.generation, r.last_generation);
@@ -2083,7 +2070,7 @@ void sssp_update_each(Context& ctx, Graph& g, const dyngb200_batch& batch, Tree*
   cudaStream_t s = ctx.stream;
   for (int i = 0; i < count; ++i)
     if (g.host_columns[trees[i]->opt.objective].dirty) graph_rescan_columns(ctx, g);
-  const StagedBatch b = stage_batch(ctx, batch, g.k);
+  const StagedBatch b = stage_batch(ctx, batch, g.k, false);
   // before the batch is applied: every objective's weights and 62-bit bound
   const int k = g.k;
   std::vector<long long> ext(2 * k + 1, 0);

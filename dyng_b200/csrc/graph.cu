@@ -883,20 +883,21 @@ __device__ void ph_mutate(const ApplyParams& p, BlockRed& R, long long tid, long
 }
 
 // ---- H: move relocated rows (live slots, in order) ---------------------------------------------
-// Which touched row a chunk of a long relocated row belongs to: the last entry whose first chunk
-// is not past it (a 32-ary search by the warp; the entries' first chunks grow with their index).
-__device__ __forceinline__ int2 find_move(const ApplyParams& p, int count, int ch) {
+// Which row a chunk of a list of long rows -- (row, its first chunk) -- belongs to: the last entry
+// whose first chunk is not past it (a 32-ary search by the warp; the entries' first chunks grow
+// with their index).
+__device__ __forceinline__ int2 find_chunk(const int2* list, int count, int ch) {
   const int lane = threadIdx.x & 31;
   int lo = 0, hi = count;
   while (hi - lo > 1) {
     const int stride = (hi - lo + 31) >> 5;
     const int probe = lo + lane * stride;
-    const bool ok = probe < hi && __ldcg(&p.move_list[probe].y) <= ch;
+    const bool ok = probe < hi && __ldcg(&list[probe].y) <= ch;
     const int last = 31 - __clz(__ballot_sync(0xffffffffu, ok));  // lane 0: list[lo].y <= ch
     lo = lo + last * stride;
     hi = min(hi, lo + stride);
   }
-  return make_int2(__ldcg(&p.move_list[lo].x), __ldcg(&p.move_list[lo].y));
+  return make_int2(__ldcg(&list[lo].x), __ldcg(&list[lo].y));
 }
 
 // The live slots of every chunk of the long relocated rows (after the tombstones of step G): each
@@ -908,7 +909,7 @@ __device__ void ph_move_count(const ApplyParams& p, long long tid, long long thr
   const int chunks = static_cast<int>(c->move_heavy & ((1ULL << 40) - 1));
   const int rows_out = c->rows_out;
   for (long long ch = tid >> 5; ch < chunks; ch += threads >> 5) {
-    const int2 at = find_move(p, count, static_cast<int>(ch));
+    const int2 at = find_chunk(p.move_list, count, static_cast<int>(ch));
     const int side = at.x < rows_out ? 0 : 1;
     const int s = side == 0 ? at.x : at.x - rows_out;
     const RowDesc desc = (side == 0 ? p.g.out_desc : p.g.in_desc)[(side == 0 ? p.rows_out : p.rows_in)[s]];
@@ -987,7 +988,7 @@ __device__ void ph_move(const ApplyParams& p, long long tid, long long threads) 
   const int count = static_cast<int>(c->move_heavy >> 40);
   const int chunks = static_cast<int>(c->move_heavy & ((1ULL << 40) - 1));
   for (long long ch = warp; ch < chunks; ch += warps) {
-    const int2 at = find_move(p, count, static_cast<int>(ch));
+    const int2 at = find_chunk(p.move_list, count, static_cast<int>(ch));
     const int side = at.x < rows_out ? 0 : 1;
     const int s = side == 0 ? at.x : at.x - rows_out;
     const int32_t r = (side == 0 ? p.rows_out : p.rows_in)[s];
@@ -1282,49 +1283,90 @@ __global__ void k_index_clear(GraphView g) {
     g.eidx[i].key = kKeyEmpty;
 }
 
-// One warp per row, the lanes over its slots: hub rows (tens of thousands of slots in R-MAT
-// graphs) do not serialise one thread.
-__global__ void k_index_out(GraphView g, long long n, unsigned* error) {
-  const int lane = threadIdx.x & 31;
+// Rows longer than this are cut into chunks of as many slots for the storage passes (index build,
+// compaction): a hub row of 200,000 slots kept one warp busy for 10 ms while the rest of the pass
+// took one.
+constexpr int kLongRow = 1024;
+struct LongRows {
+  int2* list;  // (row, its first chunk)
+  u64* count;  // rows << 40 | chunks
+  int* live;   // compaction: the live slots of every chunk
+};
+__device__ __forceinline__ int long_rows(const LongRows& l) { return static_cast<int>(*l.count >> 40); }
+__device__ __forceinline__ int long_chunks(const LongRows& l) {
+  return static_cast<int>(*l.count & ((1ULL << 40) - 1));
+}
+__global__ void k_list_long(const RowDesc* desc, long long n, LongRows l) {
+  for (long long v = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; v < n;
+       v += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const int len = desc[v].len;
+    if (len <= kLongRow) continue;
+    const u64 prev = atomicAdd(l.count, (1ULL << 40) | static_cast<u64>((len + kLongRow - 1) / kLongRow));
+    l.list[prev >> 40] = make_int2(static_cast<int>(v), static_cast<int>(prev & ((1ULL << 40) - 1)));
+  }
+}
+// Every row's slots by whole warps: `visit(v, desc, e0, e1)` for each short row, then for each
+// chunk of the long ones.
+template <typename F>
+__device__ __forceinline__ void for_rows(const RowDesc* desc, long long n, const LongRows& l, F visit) {
+  const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const long long warps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
+  for (long long v = warp; v < n; v += warps) {
+    const RowDesc d = desc[v];
+    if (d.len <= kLongRow) visit(v, d, 0, d.len);
+  }
+  const int rows = long_rows(l), chunks = long_chunks(l);
+  for (long long ch = warp; ch < chunks; ch += warps) {
+    const int2 at = find_chunk(l.list, rows, static_cast<int>(ch));
+    const RowDesc d = desc[at.x];
+    const int e0 = static_cast<int>(ch - at.y) * kLongRow;
+    visit(at.x, d, e0, min(d.len, e0 + kLongRow));
+  }
+}
+
+__global__ void k_index_out(GraphView g, long long n, LongRows l, unsigned* error) {
+  const int lane = threadIdx.x & 31;
   long long live = 0;
-  for (long long u = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; u < n;
-       u += warps) {
-    const RowDesc d = g.out_desc[u];
-    for (int e = lane; e < d.len; e += 32) {
+  bool failed = false;
+  for_rows(g.out_desc, n, l, [&](long long u, RowDesc d, int e0, int e1) {
+    if (__any_sync(0xffffffffu, failed)) return;  // a full table: no other walk of it
+    for (int e = e0 + lane; e < e1; e += 32) {
       const int32_t x = g.out_col[d.start + e];
       if (x < 0) continue;
       bool reused = false;
       const long long ie = index_insert(g, edge_key(static_cast<int32_t>(u), x), &reused);
       if (ie < 0) {
-        atomicOr(error, kErrCapacity);  // a full table: the build fails, no other walk needed
-        return;
+        atomicOr(error, kErrCapacity);  // the build fails
+        failed = true;
+        break;
       }
       g.eidx[ie].out = d.start + e;
       ++live;
     }
-  }
+    __syncwarp();
+  });
   if (live) atomicAdd(reinterpret_cast<unsigned long long*>(&g.counters->idx_live),
                       static_cast<unsigned long long>(live));
 }
 
-__global__ void k_index_in(GraphView g, long long n, unsigned* error) {
+__global__ void k_index_in(GraphView g, long long n, LongRows l, unsigned* error) {
   const int lane = threadIdx.x & 31;
-  const long long warps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
-  for (long long v = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; v < n;
-       v += warps) {
-    const RowDesc d = g.in_desc[v];
-    for (int e = lane; e < d.len; e += 32) {
+  bool failed = false;
+  for_rows(g.in_desc, n, l, [&](long long v, RowDesc d, int e0, int e1) {
+    if (__any_sync(0xffffffffu, failed)) return;
+    for (int e = e0 + lane; e < e1; e += 32) {
       const int32_t y = g.in_col[d.start + e];
       if (y < 0) continue;
       const long long ie = index_find(g, edge_key(y, static_cast<int32_t>(v)));
       if (ie < 0) {
         atomicOr(error, kErrInternal);
-        return;
+        failed = true;
+        break;
       }
       g.eidx[ie].in = d.start + e;
     }
-  }
+    __syncwarp();
+  });
 }
 
 // Compaction of one side, on the device: the live slots of every row (col >= 0), in storage
@@ -1337,35 +1379,64 @@ __device__ __forceinline__ long long row_slack(long long len, double headroom) {
   return (len + extra + 3) & ~3LL;
 }
 
+// Live slots: of a short row into its new capacity, of a long row's chunks into `l.live`.
 __global__ void k_compact_count(const RowDesc* desc, const int32_t* col, long long n,
-                                double headroom, long long* cap) {
+                                double headroom, LongRows l, long long* cap) {
   const int lane = threadIdx.x & 31;
+  const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const long long warps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
-  for (long long v = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; v < n;
-       v += warps) {
+  for (long long v = warp; v < n; v += warps) {
     const RowDesc d = desc[v];
+    if (d.len > kLongRow) continue;
     int live = 0;
     for (int e = lane; e < d.len; e += 32) live += col[d.start + e] >= 0;
-    for (int o = 16; o > 0; o >>= 1) live += __shfl_down_sync(0xffffffffu, live, o);
+    live = __reduce_add_sync(0xffffffffu, live);
     if (lane == 0) cap[v] = row_slack(live, headroom);
+  }
+  const int rows = long_rows(l), chunks = long_chunks(l);
+  for (long long ch = warp; ch < chunks; ch += warps) {
+    const int2 at = find_chunk(l.list, rows, static_cast<int>(ch));
+    const RowDesc d = desc[at.x];
+    const int e0 = static_cast<int>(ch - at.y) * kLongRow;
+    const int e1 = min(d.len, e0 + kLongRow);
+    int live = 0;
+    for (int e = e0 + lane; e < e1; e += 32) live += col[d.start + e] >= 0;
+    live = __reduce_add_sync(0xffffffffu, live);
+    if (lane == 0) l.live[ch] = live;
   }
 }
 
-__global__ void k_compact_copy(RowDesc* desc, int32_t* cap_out, int32_t* dead,
+// The capacities of the long rows from their chunks' live slots, a warp per row.
+__global__ void k_compact_long(const RowDesc* desc, double headroom, LongRows l, long long* cap) {
+  const int lane = threadIdx.x & 31;
+  const int rows = long_rows(l);
+  const long long warps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
+  for (long long q = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; q < rows;
+       q += warps) {
+    const int2 at = l.list[q];
+    const int chunks = (desc[at.x].len + kLongRow - 1) / kLongRow;
+    int live = 0;
+    for (int c = lane; c < chunks; c += 32) live += l.live[at.y + c];
+    live = __reduce_add_sync(0xffffffffu, live);
+    if (lane == 0) cap[at.x] = row_slack(live, headroom);
+  }
+}
+
+// The live slots of every row, in order, to their new places; the new descriptors go to `next`
+// (the long rows' chunks still read the old ones).
+__global__ void k_compact_copy(const RowDesc* desc, RowDesc* next, int32_t* cap_out, int32_t* dead,
                                const int32_t* col, const int32_t* w, long long old_arena,
                                const long long* start, int32_t* ncol, int32_t* nw,
-                               long long new_arena, int k, long long n) {
+                               long long new_arena, int k, long long n, LongRows l) {
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
+  const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const long long warps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
-  for (long long v = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; v < n;
-       v += warps) {
-    const RowDesc d = desc[v];
-    const long long to = start[v];
+  auto copy = [&](const RowDesc& d, long long to, int e0, int e1) {
     int at = 0;
-    for (int e0 = 0; e0 < d.len; e0 += 32) {
-      const int e = e0 + lane;
-      const int32_t x = e < d.len ? col[d.start + e] : kDead;
+    for (int base = e0; base < e1; base += 32) {
+      const int e = base + lane;
+      const int32_t x = e < e1 ? col[d.start + e] : kDead;
       const unsigned live = __ballot_sync(0xffffffffu, x >= 0);
       if (x >= 0) {
         const long long dst = to + at + __popc(live & below);
@@ -1375,12 +1446,31 @@ __global__ void k_compact_copy(RowDesc* desc, int32_t* cap_out, int32_t* dead,
       }
       at += __popc(live);
     }
-    __syncwarp();
-    if (lane == 0) {
-      desc[v] = RowDesc{static_cast<uint32_t>(to), at};
-      cap_out[v] = static_cast<int32_t>(start[v + 1] - to);
-      dead[v] = 0;
-    }
+    return at;
+  };
+  auto finish = [&](long long v, long long to, int len) {
+    if (lane != 0) return;
+    next[v] = RowDesc{static_cast<uint32_t>(to), len};
+    cap_out[v] = static_cast<int32_t>(start[v + 1] - to);
+    dead[v] = 0;
+  };
+  for (long long v = warp; v < n; v += warps) {
+    const RowDesc d = desc[v];
+    if (d.len > kLongRow) continue;
+    const long long to = start[v];
+    finish(v, to, copy(d, to, 0, d.len));
+  }
+  const int rows = long_rows(l), chunks = long_chunks(l);
+  for (long long ch = warp; ch < chunks; ch += warps) {
+    const int2 at = find_chunk(l.list, rows, static_cast<int>(ch));
+    const RowDesc d = desc[at.x];
+    int before = 0;
+    for (int q = at.y + lane; q < ch; q += 32) before += l.live[q];
+    before = __reduce_add_sync(0xffffffffu, before);
+    const long long to = start[at.x];
+    const int e0 = static_cast<int>(ch - at.y) * kLongRow;
+    const int moved = copy(d, to + before, e0, min(d.len, e0 + kLongRow));
+    if (e0 + kLongRow >= d.len) finish(at.x, to, before + moved);  // the row's last chunk
   }
 }
 
@@ -1953,6 +2043,24 @@ struct MaintenanceTimer {
 };
 }  // namespace
 
+// The long rows of one side listed on the device (`l`: reserved by reserve_long_rows).
+static LongRows list_long_rows(Context& ctx, const RowDesc* desc, long long n) {
+  Workspace& ws = ctx.ws;
+  LongRows l{reinterpret_cast<int2*>(ws.long_list.ptr), ws.long_count.ptr, ws.long_live.ptr};
+  DYNGB200_CUDA(cudaMemsetAsync(l.count, 0, sizeof(u64), ctx.stream));
+  ++ctx.launches;
+  k_list_long<<<grid_for(n, kBlock, ctx.sm_count), kBlock, 0, ctx.stream>>>(desc, n, l);
+  DYNGB200_CUDA(cudaGetLastError());
+  return l;
+}
+// At most arena / kLongRow long rows, and twice as many chunks.
+static void reserve_long_rows(Context& ctx, long long arena) {
+  const size_t rows = static_cast<size_t>(arena / kLongRow) + 1;
+  ctx.ws.long_list.reserve(2 * rows);  // int2 entries
+  ctx.ws.long_live.reserve(2 * rows);
+  ctx.ws.long_count.reserve(1);
+}
+
 // (Re)build the edge index with room for `extra` more edges and at least `min_cap` slots.
 // Slots of an edge index for the graph's edges plus `extra` insertions (load <= 1/3 after the
 // build), at least min_cap.  A rebuild comes when live plus deleted keys pass 60 %: with a third
@@ -1970,6 +2078,7 @@ void graph_index_build(Context& ctx, Graph& g, long long extra, long long min_ca
   cudaStream_t s = ctx.stream;
   Workspace& ws = ctx.ws;
   ws.ctl.reserve(1, s);  // before the index changes: every allocation comes first
+  reserve_long_rows(ctx, g.arena_cap);
   const long long want = index_want(g, extra, min_cap);
   if (want != g.ecap) {
     // the new array first: a failed allocation leaves the old index, whole, in place
@@ -1987,8 +2096,10 @@ void graph_index_build(Context& ctx, Graph& g, long long extra, long long min_ca
   const int grid = ctx.sm_count * 8;
   ctx.launches += 3;
   k_index_clear<<<grid, kBlock, 0, s>>>(v);
-  k_index_out<<<grid, kBlock, 0, s>>>(v, gc.n, &ws.ctl.ptr->error);
-  k_index_in<<<grid, kBlock, 0, s>>>(v, gc.n, &ws.ctl.ptr->error);
+  k_index_out<<<grid, kBlock, 0, s>>>(v, gc.n, list_long_rows(ctx, v.out_desc, gc.n),
+                                      &ws.ctl.ptr->error);
+  k_index_in<<<grid, kBlock, 0, s>>>(v, gc.n, list_long_rows(ctx, v.in_desc, gc.n),
+                                     &ws.ctl.ptr->error);
   DYNGB200_CUDA(cudaGetLastError());
   unsigned err = 0;
   DYNGB200_CUDA(cudaMemcpyAsync(&err, &ws.ctl.ptr->error, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
@@ -2118,14 +2229,22 @@ void graph_compact(Context& ctx, Graph& g, long long need_out, long long need_in
   const long long demand[2] = {
       std::max(0LL, need_out - static_cast<long long>(g.host_counters.out_top)),
       std::max(0LL, need_in - static_cast<long long>(g.host_counters.in_top))};
+  reserve_long_rows(ctx, g.arena_cap);
+  // the new capacity of every row of a side, from its live slots
+  auto count_rows = [&](int side) {
+    const RowDesc* desc = (side == 0 ? g.out_desc : g.in_desc).ptr;
+    const LongRows l = list_long_rows(ctx, desc, n);
+    DYNGB200_CUDA(cudaMemsetAsync(cap.ptr + n, 0, sizeof(long long), s));
+    ctx.launches += 2;
+    k_compact_count<<<grid, kBlock, 0, s>>>(desc, (side == 0 ? g.out_col : g.in_col).ptr, n,
+                                            g.props.headroom, l, cap.ptr);
+    k_compact_long<<<ctx.sm_count, kBlock, 0, s>>>(desc, g.props.headroom, l, cap.ptr);
+    DYNGB200_CUDA(cudaGetLastError());
+    return l;
+  };
   // pass 1: the new tops of both sides decide the one arena size the sides share
   for (int side = 0; side < 2; ++side) {
-    DYNGB200_CUDA(cudaMemsetAsync(cap.ptr + n, 0, sizeof(long long), s));
-    ctx.launches += 1;
-    k_compact_count<<<grid, kBlock, 0, s>>>((side == 0 ? g.out_desc : g.in_desc).ptr,
-                                            (side == 0 ? g.out_col : g.in_col).ptr, n,
-                                            g.props.headroom, cap.ptr);
-    DYNGB200_CUDA(cudaGetLastError());
+    count_rows(side);
     ctx.launches += exclusive_scan(cap.ptr, start.ptr, n + 1, temp.ptr, s);
     DYNGB200_CUDA(cudaMemcpyAsync(&top[side], start.ptr + n, sizeof(long long),
                                   cudaMemcpyDeviceToHost, s));
@@ -2138,7 +2257,9 @@ void graph_compact(Context& ctx, Graph& g, long long need_out, long long need_in
   // descriptors are rewritten in place, and both sides share arena_cap): a failed allocation
   // leaves the graph as it was
   DevBuf<int32_t> ncol[2], nw[2];
+  DevBuf<RowDesc> ndesc[2];
   for (int side = 0; side < 2; ++side) {
+    ndesc[side].reserve(static_cast<size_t>(g.n_cap));
     ncol[side].reserve(static_cast<size_t>(arena));
     nw[side].reserve(static_cast<size_t>(arena) * static_cast<size_t>(k));
   }
@@ -2149,23 +2270,28 @@ void graph_compact(Context& ctx, Graph& g, long long need_out, long long need_in
   DevBuf<EdgeSlot> index;
   if (index_cap != g.ecap) index.reserve(static_cast<size_t>(index_cap));
   ctx.ws.ctl.reserve(1, s);
+  reserve_long_rows(ctx, std::max(arena, g.arena_cap));
   for (int side = 0; side < 2; ++side) {
     DevBuf<int32_t>& col = side == 0 ? g.out_col : g.in_col;
     DevBuf<int32_t>& w = side == 0 ? g.out_w : g.in_w;
-    RowDesc* desc = (side == 0 ? g.out_desc : g.in_desc).ptr;
-    DYNGB200_CUDA(cudaMemsetAsync(cap.ptr + n, 0, sizeof(long long), s));
-    ctx.launches += 2;
-    k_compact_count<<<grid, kBlock, 0, s>>>(desc, col.ptr, n, g.props.headroom, cap.ptr);
-    ctx.launches += exclusive_scan(cap.ptr, start.ptr, n + 1, temp.ptr, s);
+    const DevBuf<RowDesc>& desc = side == 0 ? g.out_desc : g.in_desc;
+    const LongRows l = count_rows(side);
+    ctx.launches += 1 + exclusive_scan(cap.ptr, start.ptr, n + 1, temp.ptr, s);
     DYNGB200_CUDA(cudaMemsetAsync(ncol[side].ptr, 0xff,
                                   static_cast<size_t>(arena) * sizeof(int32_t), s));
-    k_compact_copy<<<grid, kBlock, 0, s>>>(desc, (side == 0 ? g.out_cap : g.in_cap).ptr,
+    // descriptors past the graph's vertices (capacity for growth) as they are
+    DYNGB200_CUDA(cudaMemcpyAsync(ndesc[side].ptr, desc.ptr, g.n_cap * sizeof(RowDesc),
+                                  cudaMemcpyDeviceToDevice, s));
+    k_compact_copy<<<grid, kBlock, 0, s>>>(desc.ptr, ndesc[side].ptr,
+                                           (side == 0 ? g.out_cap : g.in_cap).ptr,
                                            (side == 0 ? g.out_dead : g.in_dead).ptr, col.ptr,
                                            w.ptr, g.arena_cap, start.ptr, ncol[side].ptr,
-                                           nw[side].ptr, arena, g.k, n);
+                                           nw[side].ptr, arena, g.k, n, l);
     DYNGB200_CUDA(cudaGetLastError());
   }
   DYNGB200_CUDA(cudaStreamSynchronize(s));
+  g.out_desc.swap(ndesc[0]);
+  g.in_desc.swap(ndesc[1]);
   g.out_col.swap(ncol[0]);
   g.out_w.swap(nw[0]);
   g.in_col.swap(ncol[1]);

@@ -233,6 +233,8 @@ struct Workspace {
   DevBuf<int> move_list, move_live;      // long relocated rows: (row, first chunk); live slots
   DevBuf<long long> col_ins_max, col_sum_delta, col_removed_at_max, col_written_max,
       col_written_at_max;
+  DevBuf<int> long_list, long_live;  // storage passes: (row, first chunk) of the long rows
+  DevBuf<u64> long_count;
   // batch staging: a small host batch in one piece (page-locked copy, device copy, 16-byte words
   // the next control-block upload brings over with it), larger ones array by array
   HostBuf<int4> stage_host;

@@ -159,6 +159,7 @@ struct UpdateCtl {
   int rounds;
   int iterations, epochs;
   int levels;
+  int walked;           // the invalidation was the subtree walk
   long long pushes;
   long long invalidated;
   long long affected;

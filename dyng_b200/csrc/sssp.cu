@@ -798,6 +798,62 @@ __device__ __forceinline__ void clear_step(UpdateCtl* c, int it) {
   c->local_rounds[(it + 1) % 3] = 0;
 }
 
+// The invalidation without a schedule's say: a top-down walk of the invalidated subtrees where
+// the changed tree edges are few, pointer jumping otherwise.  Pointer jumping visits every vertex
+// in each of its four to seven rounds (100 us at 4.2M vertices, 29 us at a thousand); the walk
+// reads the out-rows of the invalidated vertices alone, but takes as many levels as their subtrees
+// are deep.  So it is tried on graphs of at least kWalkDegree edges per vertex (shallow trees; on
+// a grid the subtrees are thousands of levels deep) with at most kWalkRoots roots, and what is not
+// reached after kWalkLevels levels of the grid is left to pointer jumping.
+constexpr long long kWalkDegree = 6;
+constexpr long long kWalkRoots = 32;
+constexpr int kWalkPairs = 2048;  // larger batches hardly hold so few roots: not listed for it
+constexpr int kWalkLevels = 2;
+
+// A block's own levels of the walk: the subtrees below the vertices that it invalidated (a vertex
+// has one tree parent, so no two blocks meet).  What does not fit is shared with the grid.
+constexpr int kWalkLight = 256;
+constexpr int kWalkMed = 16;
+constexpr int kWalkRounds = 8;
+__device__ __forceinline__ void local_walk(const SsspParams& p, Ctx& X) {
+  __shared__ int s_own[kWalkLight + kWalkMed];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kWarps = kThreads / 32;
+  for (int round = 0;; ++round) {
+    __syncthreads();
+    const int nl = g_stage.cnt[kStNext], nm = g_stage.cnt[kStNextMed];
+    if (nl + nm == 0 || nl > kWalkLight || nm > kWalkMed || round >= kWalkRounds) return;
+    if (static_cast<int>(threadIdx.x) < nl) s_own[threadIdx.x] = g_stage.data[kStNext][threadIdx.x];
+    if (static_cast<int>(threadIdx.x) < nm)
+      s_own[kWalkLight + threadIdx.x] = g_stage.data[kStNextMed][threadIdx.x];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      g_stage.cnt[kStNext] = 0;
+      g_stage.cnt[kStNextMed] = 0;
+    }
+    __syncthreads();
+    const int per = (nl + kWarps - 1) / kWarps;
+    static_assert(kWalkLight <= 32 * kWarps && kWalkLight <= kThreads, "one row per lane");
+    if (warp * per < nl) {
+      const int i = warp * per + lane;
+      int owner = -1;
+      RowDesc desc{0, 0};
+      if (lane < per && i < nl) {
+        owner = s_own[i];
+        ++X.rows;
+        desc = p.g.out_desc[owner];
+      }
+      warp_rows<kWalk>(p, X, owner, 0, desc.start, desc.len);
+    }
+    for (int i = warp; i < nm; i += kWarps) {
+      const int owner = s_own[kWalkLight + i];
+      const RowDesc desc = p.g.out_desc[owner];
+      if (lane == 0) ++X.rows;
+      warp_slots<kWalk>(p, X, owner, 0, desc.start, 0, desc.len);
+    }
+  }
+}
+
 // The near-far loop (fused.cuh:288-417) run by the whole grid.  Returns false on a timeout.
 __device__ bool near_far(const SsspParams& p, Ctx& X, LoopState& S, unsigned& bar, u64 delta,
                          long long n, int small) {
@@ -1020,6 +1076,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
         p.packed[v] = kPackedInf;
       }
     }
+    const bool may_walk = p.walk || (p.tree_trusted && c->pairs <= kWalkPairs &&
+                                     p.g.counters->m >= kWalkDegree * n);
     // ---- roots: heads v of changed edges (u,v) with parent[v] == u ---------------------------
     const int pairs = c->pairs;
     int changed = 0;
@@ -1039,7 +1097,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
           invalidate(p, static_cast<int>(v));
           ++w_inval;
           changed = 2;
-          if (p.walk) {
+          if (may_walk) {
             const ListSet W0{p.near_a, &c->walk_cnt[0], p.near_med_a, &c->walk_med_cnt[0],
                              p.heavy_a, &c->walk_heavy[0], kStNext, kStNextMed, nullptr, 0};
             list_append(W0, v, p.g.out_desc[v].len, p.heavy_degree);
@@ -1061,7 +1119,55 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
     // edge changed, so that a parent cycle is still reported as the reference reports it
     const int changed_bits = ld_cg(&c->changed);
     const bool any_changed = (changed_bits & 2) || (!p.tree_trusted && (changed_bits & 1));
-    if (!p.walk) {
+    bool walked = p.walk != 0;
+    if (!walked && may_walk) {
+      const long long roots = static_cast<long long>(ld_cg(&c->walk_cnt[0])) + ld_cg(&c->walk_med_cnt[0]) +
+                              static_cast<long long>(ld_cg(&c->walk_heavy[0]) >> 40);
+      walked = roots <= kWalkRoots;
+    }
+    if (walked) {
+      // ---- subtree invalidation by a walk down the old tree's edges, level by level ---------
+      X.gen = gen_inv;
+      int level = 0;
+      while (true) {
+        const int cs = level % 3;
+        const int nc = ld_cg(&c->walk_cnt[cs]);
+        const int mc = ld_cg(&c->walk_med_cnt[cs]);
+        const u64 hc = ld_cg(&c->walk_heavy[cs]);
+        if (nc == 0 && mc == 0 && (hc >> 40) == 0) break;
+        if (!p.walk && level >= kWalkLevels) {
+          // too deep: pointer jumping finishes it
+          walked = false;
+          break;
+        }
+        if (level > n + 1) {
+          if (tid == 0) atomicOr(&c->error, kErrNotConverged);
+          break;
+        }
+        const int nb = (level + 1) & 1;
+        X.next = ListSet{nb ? p.near_b : p.near_a, &c->walk_cnt[(level + 1) % 3],
+                         nb ? p.near_med_b : p.near_med_a, &c->walk_med_cnt[(level + 1) % 3],
+                         nb ? p.heavy_b : p.heavy_a, &c->walk_heavy[(level + 1) % 3], kStNext,
+                         kStNextMed, nullptr, 0};
+        if (tid == 0) {
+          c->walk_cnt[(level + 2) % 3] = 0;
+          c->walk_med_cnt[(level + 2) % 3] = 0;
+          c->walk_heavy[(level + 2) % 3] = 0;
+        }
+        const int cb = level & 1;
+        expand<kWalk>(p, X, cb ? p.near_b : p.near_a, nc, cb ? p.near_med_b : p.near_med_a, mc,
+                      cb ? p.heavy_b : p.heavy_a, hc, gwarp, nwarps);
+        local_walk(p, X);
+        if (!grid_barrier(c, bar)) return;
+        ++level;
+      }
+      w_inval += X.appends;
+      walk_rows = X.rows;
+      walk_slots = X.slots;
+      X.appends = X.rows = X.slots = 0;
+      if (tid == 0) c->levels = level;
+    }
+    if (!walked) {
       // ---- subtree invalidation by pointer jumping (fused.cuh:199-234) ------------------------
       // ancestor[v]: >= 0 the current ancestor, -1 the chain ended without a root, kMarked:
       // invalidated.  Invariant: ancestor[x] >= 0 implies no root on the tree path from x up to
@@ -1241,45 +1347,10 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
           }
         }
       }
-      if (tid == 0) c->phase_ns[2] = global_ns();
-    } else {
-      // ---- subtree invalidation by a walk down the old tree's edges, level by level ---------
-      X.gen = gen_inv;
-      int level = 0;
-      while (true) {
-        const int cs = level % 3;
-        const int nc = ld_cg(&c->walk_cnt[cs]);
-        const int mc = ld_cg(&c->walk_med_cnt[cs]);
-        const u64 hc = ld_cg(&c->walk_heavy[cs]);
-        if (nc == 0 && mc == 0 && (hc >> 40) == 0) break;
-        if (level > n + 1) {
-          if (tid == 0) atomicOr(&c->error, kErrNotConverged);
-          break;
-        }
-        const int nb = (level + 1) & 1;
-        X.next = ListSet{nb ? p.near_b : p.near_a, &c->walk_cnt[(level + 1) % 3],
-                         nb ? p.near_med_b : p.near_med_a, &c->walk_med_cnt[(level + 1) % 3],
-                         nb ? p.heavy_b : p.heavy_a, &c->walk_heavy[(level + 1) % 3], kStNext,
-                         kStNextMed, nullptr, 0};
-        if (tid == 0) {
-          c->walk_cnt[(level + 2) % 3] = 0;
-          c->walk_med_cnt[(level + 2) % 3] = 0;
-          c->walk_heavy[(level + 2) % 3] = 0;
-        }
-        const int cb = level & 1;
-        expand<kWalk>(p, X, cb ? p.near_b : p.near_a, nc, cb ? p.near_med_b : p.near_med_a, mc,
-                      cb ? p.heavy_b : p.heavy_a, hc, gwarp, nwarps);
-        if (!grid_barrier(c, bar)) return;
-        ++level;
-      }
-      w_inval += X.appends;
-      walk_rows = X.rows;
-      walk_slots = X.slots;
-      X.appends = X.rows = X.slots = 0;
-      if (tid == 0) {
-        c->levels = level;
-        c->phase_ns[2] = global_ns();
-      }
+    }
+    if (tid == 0) {
+      c->phase_ns[2] = global_ns();
+      c->walked = walked;
     }
     // The lists and stamps of the invalidation are complete (its last step ended in a barrier).
     // ---- insertion heads: pulled, or (canonical trees) offered the inserted edge ----------------
@@ -1860,7 +1931,7 @@ static void finish_tree(Context& ctx, Graph& g, Tree& t, const UpdateCtl& r, int
     st->grid_blocks = operators ? operators_grid(ctx)
                                 : (r.active_blocks > 0 && r.active_blocks < blocks ? r.active_blocks
                                                                                    : blocks);
-    st->invalidation = (r.sched_walk && t.trusted) ? 1 : 0;
+    st->invalidation = (operators ? r.sched_walk && t.trusted : r.walked != 0) ? 1 : 0;
     st->apply_ms = apply_ms;
     st->sssp_ms = sssp_ms;
     st->rounds = r.rounds;

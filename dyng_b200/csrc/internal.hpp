@@ -503,6 +503,11 @@ void sssp_update_end(PendingUpdate& u, dyngb200_stats* st);
 // (occupancy x SMs, or Context::max_update_blocks when smaller).
 int update_blocks_per_sm(Context& ctx);
 int update_grid_blocks(Context& ctx);
+// The blocks of an sssp launch on a graph of n vertices: a barrier of the whole grid costs 2.2 us,
+// one of a few blocks 1.2, and a small graph keeps no more than a block per 384 vertices busy
+// (measured, sssp kernel of an update: 1,024 vertices 54 us with 444 blocks, 49 with 4; 12,345
+// vertices 113 us, 101 with 32; 65,536 vertices 127 us, 119 with 148; no gain from 260,000 on).
+int update_blocks_for(Context& ctx, long long n);
 void sssp_update_each(Context& ctx, Graph& g, const dyngb200_batch& batch, Tree* const* trees,
                       int count, dyngb200_stats* stats);
 void graph_apply(Context& ctx, Graph& g, const dyngb200_batch& batch,

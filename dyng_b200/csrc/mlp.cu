@@ -413,7 +413,7 @@ void learned_infer_args(Context& ctx, Tree& t, const Scheduler* sch, InferArgs* 
   a.w = sch ? sch->wbf16.ptr : nullptr;
   if (sch) a.nrm = norm_of(*sch);
   a.hist = t.hist.ptr;
-  a.blocks = update_grid_blocks(ctx);
+  a.blocks = update_blocks_for(ctx, t.n);
   *out = a;
 }
 

@@ -1639,9 +1639,15 @@ void schedule_into(const dyngb200_schedule& sched, UpdateCtl& init) {
   init.active_blocks = sched.grid_blocks > 0 ? sched.grid_blocks : 0;
 }
 
-static int persistent_blocks(Context& ctx, const dyngb200_schedule& sched) {
-  (void)sched;  // the schedule's grid size is applied on the device (active_blocks)
-  return update_grid_blocks(ctx);
+int update_blocks_for(Context& ctx, long long n) {
+  constexpr long long kVertices = 384;
+  return static_cast<int>(std::min<long long>(update_grid_blocks(ctx),
+                                              std::max(4LL, (n + kVertices - 1) / kVertices)));
+}
+
+static int persistent_blocks(Context& ctx, const dyngb200_schedule& sched, long long n) {
+  // a schedule's own grid size is applied on the device (active_blocks)
+  return sched.grid_blocks > 0 ? update_grid_blocks(ctx) : update_blocks_for(ctx, n);
 }
 
 void require_intact(const Graph& g) {
@@ -1756,7 +1762,7 @@ void sssp_compute(Context& ctx, Graph& g, Tree& t, dyngb200_stats* st) {
   p.generation = ws.next_generation(1, s);
   p.touch_gen = 1;
   p.heavy_degree = 256;
-  const int blocks = persistent_blocks(ctx, sched);
+  const int blocks = persistent_blocks(ctx, sched, g.n);
   cudaEvent_t e0, e1;
   DYNGB200_CUDA(cudaEventCreate(&e0));
   DYNGB200_CUDA(cudaEventCreate(&e1));
@@ -1872,7 +1878,7 @@ void sssp_update_begin(Context& ctx, Graph& g, Tree& t, const dyngb200_batch& ba
   if (g.host_columns[t.opt.objective].dirty) graph_rescan_columns(ctx, g);
   graph_index_reserve(ctx, g, batch.num_insertions * (g.props.directed ? 1 : 2));
   u.b = stage_batch(ctx, batch, g.k, true);
-  u.blocks = persistent_blocks(ctx, sched);
+  u.blocks = persistent_blocks(ctx, sched, g.n);
   for (cudaEvent_t& e : ctx.update_events)
     if (!e) DYNGB200_CUDA(cudaEventCreate(&e));
   u.e0 = ctx.update_events[0];
@@ -2096,7 +2102,7 @@ static void sssp_rerun(Context& ctx, Graph& g, Tree& t, const UpdateCtl& applied
   DYNGB200_CUDA(cudaEventCreate(&e1));
   DYNGB200_CUDA(cudaEventCreate(&e2));
   upload_control(ctx, init);
-  const int blocks = persistent_blocks(ctx, sched);
+  const int blocks = persistent_blocks(ctx, sched, g.n);
   SsspParams p = base_params(ctx, g, t);
   p.from_scratch = 0;
   p.tree_n = t.n;

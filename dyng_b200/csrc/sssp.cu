@@ -269,17 +269,32 @@ __device__ __forceinline__ void visit(const SsspParams& p, Ctx& X, int owner, u6
   }
 }
 
-// The pull's offer of in-neighbour y over an in-slot of weight w: packed (d(y) + w, y), or INF.
-__device__ __forceinline__ u64 pull_candidate(const SsspParams& p, Ctx& X, int y, int w) {
-  ++X.slots;
-  if (y < 0) return kPackedInf;
-  // the source's word is distance 0 for good: no load (it is the hottest address of a pull)
-  const u64 word = y == p.source ? 0 : ld_cg(&p.packed[y]);
-  ++X.words;
-  if (word == kPackedInf) return kPackedInf;
-  const u64 nd = (y == p.source ? 0 : X.pk.dist(word)) + static_cast<u64>(w);
-  if (nd > X.maxd) return kPackedInf;
-  return X.pk.pack(nd, y);
+constexpr int kNoSlot = -2;  // past the row's end (kDead: a tombstone)
+
+// The pull's offers of in-neighbours y[] over in-slots of weight w[]: packed (d(y) + w, y), or INF.
+// The neighbours' words are loaded together (one round trip for all of a lane's slots).
+template <int N>
+__device__ __forceinline__ u64 pull_candidates(const SsspParams& p, Ctx& X, const int (&y)[N],
+                                               const int (&w)[N], u64 (&out)[N]) {
+  u64 word[N];
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    // the source's word is distance 0 for good: no load (it is the hottest address of a pull)
+    word[q] = y[q] == p.source ? 0 : kPackedInf;
+    if (y[q] >= 0 && y[q] != p.source) word[q] = ld_cg(&p.packed[y[q]]);
+  }
+  u64 best = kPackedInf;
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    X.slots += y[q] >= kDead;
+    X.words += y[q] >= 0;
+    out[q] = kPackedInf;
+    if (word[q] == kPackedInf) continue;
+    const u64 nd = (y[q] == p.source ? 0 : X.pk.dist(word[q])) + static_cast<u64>(w[q]);
+    if (nd <= X.maxd) out[q] = X.pk.pack(nd, y[q]);
+    best = min(best, out[q]);
+  }
+  return best;
 }
 
 // The best offer of a pull for `owner`: keep it if smaller; on a distance decrease the owner
@@ -394,10 +409,11 @@ __device__ __forceinline__ void warp_slots(const SsspParams& p, Ctx& X, int owne
       const int e = grp << 2;
       const int4 c4 = __ldg(reinterpret_cast<const int4*>(col + e));
       const int4 w4 = __ldg(reinterpret_cast<const int4*>(wt + e));
-      if (e + 0 < e1) best = min(best, pull_candidate(p, X, c4.x, w4.x));
-      if (e + 1 < e1) best = min(best, pull_candidate(p, X, c4.y, w4.y));
-      if (e + 2 < e1) best = min(best, pull_candidate(p, X, c4.z, w4.z));
-      if (e + 3 < e1) best = min(best, pull_candidate(p, X, c4.w, w4.w));
+      const int y[4] = {e + 0 < e1 ? c4.x : kNoSlot, e + 1 < e1 ? c4.y : kNoSlot,
+                        e + 2 < e1 ? c4.z : kNoSlot, e + 3 < e1 ? c4.w : kNoSlot};
+      const int w[4] = {w4.x, w4.y, w4.z, w4.w};
+      u64 offers[4];
+      best = min(best, pull_candidates<4>(p, X, y, w, offers));
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, off));
@@ -484,34 +500,63 @@ __device__ __forceinline__ void warp_rows(const SsspParams& p, Ctx& X, int owner
     }
     return;
   }
-  for (int base = 0; base < total; base += 32) {
-    const int e = base + lane;
+  // the lane that owns slot e of the concatenated rows
+  auto owner_of = [&](int e) {
     int j = 0;
 #pragma unroll
     for (int step = 16; step > 0; step >>= 1) {
       const int cand = j + step;
       if (__shfl_sync(0xffffffffu, excl, cand) <= e) j = cand;
     }
+    return j;
+  };
+  if (MODE == kPull) {
+    // kPullSlots slots per lane and step, their loads issued together
+    constexpr int kPullSlots = 4;
+    for (int base = 0; base < total; base += 32 * kPullSlots) {
+      int j[kPullSlots], y[kPullSlots], w[kPullSlots];
+#pragma unroll
+      for (int q = 0; q < kPullSlots; ++q) {
+        const int e = base + 32 * q + lane;
+        j[q] = owner_of(e);
+        const unsigned s = __shfl_sync(0xffffffffu, start, j[q]);
+        const int ex = __shfl_sync(0xffffffffu, excl, j[q]);
+        y[q] = kNoSlot;
+        w[q] = 0;
+        if (e < total) {
+          y[q] = col[s + static_cast<unsigned>(e - ex)];
+          w[q] = wt[s + static_cast<unsigned>(e - ex)];
+        }
+      }
+      u64 offers[kPullSlots];
+      pull_candidates<kPullSlots>(p, X, y, w, offers);
+#pragma unroll
+      for (int q = 0; q < kPullSlots; ++q) {
+        if (base + 32 * q >= total) break;  // the same for the whole warp
+        // the lanes of one owner are contiguous: a segmented minimum, then one offer per owner
+        u64 best = offers[q];
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+          const u64 other = __shfl_down_sync(0xffffffffu, best, off);
+          const int oj = __shfl_down_sync(0xffffffffu, j[q], off);
+          if (lane + off < 32 && oj == j[q]) best = min(best, other);
+        }
+        const int pj = __shfl_up_sync(0xffffffffu, j[q], 1);
+        const int o = __shfl_sync(0xffffffffu, owner, j[q]);
+        if (base + 32 * q + lane < total && (lane == 0 || pj != j[q]) && best != kPackedInf)
+          offer_owner(p, X, o, best);
+      }
+    }
+    return;
+  }
+  for (int base = 0; base < total; base += 32) {
+    const int e = base + lane;
+    const int j = owner_of(e);
     const int o = __shfl_sync(0xffffffffu, owner, j);
     const u64 d = __shfl_sync(0xffffffffu, odu, j);
     const unsigned s = __shfl_sync(0xffffffffu, start, j);
     const int ex = __shfl_sync(0xffffffffu, excl, j);
-    if (MODE == kPull) {
-      // the lanes of one owner are contiguous: a segmented minimum, then one offer per owner
-      u64 best = kPackedInf;
-      if (e < total) {
-        const unsigned slot = s + static_cast<unsigned>(e - ex);
-        best = pull_candidate(p, X, col[slot], wt[slot]);
-      }
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const u64 other = __shfl_down_sync(0xffffffffu, best, off);
-        const int oj = __shfl_down_sync(0xffffffffu, j, off);
-        if (lane + off < 32 && oj == j) best = min(best, other);
-      }
-      const int pj = __shfl_up_sync(0xffffffffu, j, 1);
-      if (e < total && (lane == 0 || pj != j) && best != kPackedInf) offer_owner(p, X, o, best);
-    } else if (e < total) {
+    if (e < total) {
       const unsigned slot = s + static_cast<unsigned>(e - ex);
       visit<MODE>(p, X, o, d, col[slot], MODE == kWalk ? 0 : wt[slot]);
     }

@@ -451,10 +451,38 @@ __device__ void ph_match(const ApplyParams& p, long long tid, long long threads)
   }
 }
 
+// Multigraph rows are read by a warp 128 slots at a time, four consecutive ones per lane (rows
+// start on 16-byte boundaries and own whole groups of four).  With one slot per lane and step a
+// pair on a hub row of 10,000 slots took 300 dependent loads: 53 us of a 1,000-change step.
+constexpr int kScanSlots = 128;
+// This lane's matches among slots [base + 4 lane, base + 4 lane + 4) of a row, as four bits.
+__device__ __forceinline__ unsigned row_matches(const int32_t* col, int base, int len, int32_t want) {
+  const int e = base + 4 * (threadIdx.x & 31);
+  if (e >= len) return 0;
+  const int4 c = *reinterpret_cast<const int4*>(col + e);
+  unsigned m = c.x == want ? 1u : 0u;
+  if (e + 1 < len && c.y == want) m |= 2u;
+  if (e + 2 < len && c.z == want) m |= 4u;
+  if (e + 3 < len && c.w == want) m |= 8u;
+  return m;
+}
+// Matches in the lanes below this one (all lanes call); *all receives the warp's.
+__device__ __forceinline__ int matches_before(unsigned m, int* all) {
+  const int lane = threadIdx.x & 31;
+  int incl = __popc(m);
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  *all = __shfl_sync(0xffffffffu, incl, 31);
+  return incl - __popc(m);
+}
+
 // Multi-edge graphs: one thread per pair walks its rows in order (the first alive matches).
 // Records c, the first match and the match the insertions address (see resolve).
 __device__ void ph_scan_multi(const ApplyParams& p, long long tid, long long threads) {
-  // one warp per pair: the lanes read a row 32 slots at a time, the matches ranked by a ballot
+  // one warp per pair: the lanes read a row kScanSlots at a time and rank the matches
   UpdateCtl* c = p.ctl;
   const int pairs = c->pairs;
   const int lane = threadIdx.x & 31;
@@ -477,30 +505,34 @@ __device__ void ph_scan_multi(const ApplyParams& p, long long tid, long long thr
       }
       const RowDesc desc = (side == 0 ? p.g.out_desc : p.g.in_desc)[r];
       const int32_t* col = (side == 0 ? p.g.out_col : p.g.in_col) + desc.start;
-      // first match, and match number d (the first survivor of the deletions); absolute slots
+      // first match, and match number d (the first survivor of the deletions); slots of the row
       int count = 0, first = -1, target = -1;
-      for (int base = 0; base < desc.len; base += 32) {
-        const int e = base + lane;
-        const unsigned ballot = __ballot_sync(0xffffffffu, e < desc.len && col[e] == want);
-        if (ballot == 0) continue;
-        if (first < 0) first = static_cast<int>(desc.start) + base + __ffs(ballot) - 1;
-        const int found = __popc(ballot);
-        if (target < 0 && d >= count && d < count + found) {
-          unsigned rest = ballot;
-          for (int k = d - count; k > 0; --k) rest &= rest - 1;  // drop the lower matches
-          target = static_cast<int>(desc.start) + base + __ffs(rest) - 1;
+      for (int base = 0; base < desc.len; base += kScanSlots) {
+        const unsigned m = row_matches(col, base, desc.len, want);
+        if (!__any_sync(0xffffffffu, m)) continue;
+        int found = 0;
+        const int before = count + matches_before(m, &found);
+        // the lane that holds the first match, and the one that holds number d
+        int mine_first = -1, mine_target = -1, rank = before;
+        for (unsigned rest = m; rest; rest &= rest - 1, ++rank) {
+          const int at = base + 4 * lane + __ffs(rest) - 1;
+          if (rank == 0) mine_first = at;
+          if (rank == d) mine_target = at;
         }
+        first = max(first, __reduce_max_sync(0xffffffffu, mine_first));
+        target = max(target, __reduce_max_sync(0xffffffffu, mine_target));
         count += found;
       }
+      auto absolute = [&](int at) { return at < 0 ? -1 : static_cast<int>(desc.start + at); };
       if (lane == 0) {
         if (side == 0) {
           p.out_count[slot] = count;
-          p.out_pos[slot] = first;
-          p.out_pos2[slot] = target;
+          p.out_pos[slot] = absolute(first);
+          p.out_pos2[slot] = absolute(target);
         } else {
           p.in_count[slot] = count;
-          p.in_pos[slot] = first;
-          p.in_pos2[slot] = target;
+          p.in_pos[slot] = absolute(first);
+          p.in_pos2[slot] = absolute(target);
         }
       }
     }
@@ -779,8 +811,8 @@ __device__ __forceinline__ void commit_add(long long t, long long* target) {
 
 // ---- G: tombstones and upserts in place -------------------------------------------------------
 // Simple graphs: one thread per pair, the matching slots from the edge index.  Multigraphs: one
-// warp per pair walking both rows in order (lanes over 32 slots at a time, the matches ranked by
-// a ballot), so a hub row is read once, coalesced, instead of slot by slot by one thread.
+// warp per pair walking both rows in order (kScanSlots at a time), so a hub row is read once,
+// coalesced, instead of slot by slot by one thread.
 __device__ void ph_mutate(const ApplyParams& p, BlockRed& R, long long tid, long long threads) {
   UpdateCtl* c = p.ctl;
   const int pairs = c->pairs;
@@ -842,15 +874,16 @@ __device__ void ph_mutate(const ApplyParams& p, BlockRed& R, long long tid, long
       const RowDesc desc = (side == 0 ? p.g.out_desc : p.g.in_desc)[r];
       int32_t* col = (side == 0 ? p.g.out_col : p.g.in_col) + desc.start;
       int32_t* w = (side == 0 ? p.g.out_w : p.g.in_w) + desc.start;
-      // multi-edge graphs: the row in order, 32 slots per step; a match's rank is the number of
+      // multi-edge graphs: the row in order, kScanSlots per step; a match's rank is the number of
       // matches before it (the first `tomb` become tombstones, rank `target` takes the upsert)
       int seen = 0;
-      for (int base = 0; base < desc.len && seen < cnt; base += 32) {
-        const int e = base + lane;
-        const bool match = e < desc.len && col[e] == want;
-        const unsigned ballot = __ballot_sync(0xffffffffu, match);
-        if (match) {
-          const int rank = seen + __popc(ballot & ((1u << lane) - 1));
+      for (int base = 0; base < desc.len && seen < cnt; base += kScanSlots) {
+        const unsigned m = row_matches(col, base, desc.len, want);
+        if (!__any_sync(0xffffffffu, m)) continue;
+        int found = 0;
+        int rank = seen + matches_before(m, &found);
+        for (unsigned rest = m; rest; rest &= rest - 1, ++rank) {
+          const int e = base + 4 * lane + __ffs(rest) - 1;
           if (rank < tomb) {
             col[e] = kDead;
             if (side == 0)
@@ -867,7 +900,7 @@ __device__ void ph_mutate(const ApplyParams& p, BlockRed& R, long long tid, long
             }
           }
         }
-        seen += __popc(ballot);
+        seen += found;
       }
     }
   }

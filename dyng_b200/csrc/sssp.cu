@@ -207,69 +207,27 @@ struct Ctx {
   unsigned tries;  // atomicMin attempts on packed words (successful or not)
 };
 
-// One slot of a row.  push: owner u relaxes (u -> y); pull: in-neighbour y offers to the owner;
-// walk: y is invalidated if its old parent is the owner.
-template <int MODE>
-__device__ __forceinline__ void visit(const SsspParams& p, Ctx& X, int owner, u64 odu, int y,
-                                      int w) {
-  ++X.slots;
-  if (y < 0) return;  // tombstone
-  if (MODE == kWalk) {
-    if (y < p.tree_n && p.parent[y] == owner && claim(p.stamp, y, X.gen)) {
-      p.packed[y] = kPackedInf;
-      touch(p, y);
-      add_candidate(p, y);
-      ++X.appends;
-      list_append(X.next, y, p.g.out_desc[y].len, p.heavy_degree);
-    }
-    return;
-  }
-  int src, dst;
-  u64 du;
-  if (MODE == kPush) {
-    if (y == p.source) return;
-    src = owner;
-    dst = y;
-    du = odu;
-  } else {
-    // the source's word is distance 0 for good: no load (it is the hottest address of a pull)
-    const u64 word = y == p.source ? 0 : ld_cg(&p.packed[y]);
-    ++X.words;
-    if (word == kPackedInf) return;
-    src = y;
-    dst = owner;
-    du = y == p.source ? 0 : X.pk.dist(word);
-  }
-  const u64 nd = du + static_cast<u64>(w);
-  if (nd > X.maxd) return;
-  const u64 cand = X.pk.pack(nd, src);
-  if (MODE == kPush) ++X.words;
-  if (cand >= ld_cg(&p.packed[dst])) return;
-  ++X.tries;
-  const u64 old = atomicMin(&p.packed[dst], cand);
-  if (cand < old) {
-    ++X.atomics;
-    touch(p, dst);
-  }
-  if (nd < X.pk.dist(old)) {
-    if (MODE == kPull) {
-      if (claim(p.stamp, dst, X.gen)) {
-        ++X.appends;
-        staged_append(kStNext, X.next.light, X.next.light_cnt, dst);
-      }
-    } else if (nd < X.threshold) {
-      if (claim(p.stamp, dst, X.gen)) {
-        ++X.appends;
-        list_append(X.next, dst, p.g.out_desc[dst].len, p.heavy_degree);
-      }
-    } else if (atomicExch(&p.in_far[dst], 1) == 0) {
-      ++X.appends;
-      staged_append(kStFar, X.far, X.far_cnt, dst);
-    }
+constexpr int kNoSlot = -2;  // past the row's end (kDead: a tombstone)
+
+// Slots y[] of rows of owner[] in the walk: y is invalidated if its old parent is the owner.  The
+// parents are loaded together (one round trip for all of a lane's slots).
+template <int N>
+__device__ __forceinline__ void walk_visit(const SsspParams& p, Ctx& X, const int (&owner)[N],
+                                           const int (&y)[N]) {
+  int parent[N];
+#pragma unroll
+  for (int q = 0; q < N; ++q) parent[q] = y[q] >= 0 && y[q] < p.tree_n ? p.parent[y[q]] : -1;
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    X.slots += y[q] >= kDead;
+    if (y[q] < 0 || parent[q] != owner[q] || !claim(p.stamp, y[q], X.gen)) continue;
+    p.packed[y[q]] = kPackedInf;
+    touch(p, y[q]);
+    add_candidate(p, y[q]);
+    ++X.appends;
+    list_append(X.next, y[q], p.g.out_desc[y[q]].len, p.heavy_degree);
   }
 }
-
-constexpr int kNoSlot = -2;  // past the row's end (kDead: a tombstone)
 
 // The pull's offers of in-neighbours y[] over in-slots of weight w[]: packed (d(y) + w, y), or INF.
 // The neighbours' words are loaded together (one round trip for all of a lane's slots).
@@ -437,11 +395,10 @@ __device__ __forceinline__ void warp_slots(const SsspParams& p, Ctx& X, int owne
   for (int grp = (e0 >> 2) + lane; grp < g1; grp += 32) {
     const int e = grp << 2;
     const int4 c4 = __ldg(reinterpret_cast<const int4*>(col + e));
-    const int4 w4 = MODE == kWalk ? make_int4(0, 0, 0, 0) : __ldg(reinterpret_cast<const int4*>(wt + e));
-    if (e + 0 < e1) visit<MODE>(p, X, owner, odu, c4.x, w4.x);
-    if (e + 1 < e1) visit<MODE>(p, X, owner, odu, c4.y, w4.y);
-    if (e + 2 < e1) visit<MODE>(p, X, owner, odu, c4.z, w4.z);
-    if (e + 3 < e1) visit<MODE>(p, X, owner, odu, c4.w, w4.w);
+    const int owners[4] = {owner, owner, owner, owner};
+    const int y[4] = {e + 0 < e1 ? c4.x : kNoSlot, e + 1 < e1 ? c4.y : kNoSlot,
+                      e + 2 < e1 ? c4.z : kNoSlot, e + 3 < e1 ? c4.w : kNoSlot};
+    walk_visit<4>(p, X, owners, y);
   }
 }
 
@@ -549,17 +506,19 @@ __device__ __forceinline__ void warp_rows(const SsspParams& p, Ctx& X, int owner
     }
     return;
   }
-  for (int base = 0; base < total; base += 32) {
-    const int e = base + lane;
-    const int j = owner_of(e);
-    const int o = __shfl_sync(0xffffffffu, owner, j);
-    const u64 d = __shfl_sync(0xffffffffu, odu, j);
-    const unsigned s = __shfl_sync(0xffffffffu, start, j);
-    const int ex = __shfl_sync(0xffffffffu, excl, j);
-    if (e < total) {
-      const unsigned slot = s + static_cast<unsigned>(e - ex);
-      visit<MODE>(p, X, o, d, col[slot], MODE == kWalk ? 0 : wt[slot]);
+  constexpr int kWalkSlots = 4;
+  for (int base = 0; base < total; base += 32 * kWalkSlots) {
+    int o[kWalkSlots], y[kWalkSlots];
+#pragma unroll
+    for (int q = 0; q < kWalkSlots; ++q) {
+      const int e = base + 32 * q + lane;
+      const int j = owner_of(e);
+      o[q] = __shfl_sync(0xffffffffu, owner, j);
+      const unsigned s = __shfl_sync(0xffffffffu, start, j);
+      const int ex = __shfl_sync(0xffffffffu, excl, j);
+      y[q] = e < total ? col[s + static_cast<unsigned>(e - ex)] : kNoSlot;
     }
+    walk_visit<kWalkSlots>(p, X, o, y);
   }
 }
 
@@ -848,11 +807,14 @@ __device__ __forceinline__ void clear_step(UpdateCtl* c, int it) {
 // in each of its four to seven rounds (100 us at 4.2M vertices, 29 us at a thousand); the walk
 // reads the out-rows of the invalidated vertices alone, but takes as many levels as their subtrees
 // are deep.  So it is tried on graphs of at least kDenseDegree edges per vertex (shallow trees; on
-// a grid the subtrees are thousands of levels deep) with at most kWalkRoots roots, and what is not
-// reached after kWalkLevels levels of the grid is left to pointer jumping.
-constexpr long long kWalkRoots = 32;
+// a grid the subtrees are thousands of levels deep) with few roots, and what is not reached after
+// two levels of the grid (six on large graphs, where a round of pointer jumping costs more) is left
+// to pointer jumping.  At R-MAT scale 22 / 1k changes the walk took 8 us in the direction that
+// invalidates 190 vertices and 138 in the one that invalidates 660, pointer jumping 107 in both.
+constexpr long long kWalkRoots = 32;      // or one per kWalkShare vertices where that is more
+constexpr long long kWalkShare = 16384;
+constexpr long long kWalkLarge = 1 << 20;  // six levels from here on, two below
 constexpr int kWalkPairs = 2048;  // larger batches hardly hold so few roots: not listed for it
-constexpr int kWalkLevels = 2;
 
 // A block's own levels of the walk: the subtrees below the vertices that it invalidated (a vertex
 // has one tree parent, so no two blocks meet).  What does not fit is shared with the grid.
@@ -1167,7 +1129,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
     if (!walked && may_walk) {
       const long long roots = static_cast<long long>(ld_cg(&c->walk_cnt[0])) + ld_cg(&c->walk_med_cnt[0]) +
                               static_cast<long long>(ld_cg(&c->walk_heavy[0]) >> 40);
-      walked = roots <= kWalkRoots;
+      walked = roots <= max(kWalkRoots, n / kWalkShare);
     }
     if (walked) {
       // ---- subtree invalidation by a walk down the old tree's edges, level by level ---------
@@ -1179,7 +1141,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
         const int mc = ld_cg(&c->walk_med_cnt[cs]);
         const u64 hc = ld_cg(&c->walk_heavy[cs]);
         if (nc == 0 && mc == 0 && (hc >> 40) == 0) break;
-        if (!p.walk && level >= kWalkLevels) {
+        if (!p.walk && level >= (n >= kWalkLarge ? 6 : 2)) {
           // too deep: pointer jumping finishes it
           walked = false;
           break;

@@ -222,7 +222,9 @@ __global__ void k_mosp_costs_init(GraphView g, long long n, const int32_t* cpar,
 
 __global__ void k_mosp_costs_jump(long long n, int columns, const int64_t* acc_in,
                                   const int32_t* anc_in, int64_t* acc_out, int32_t* anc_out,
-                                  int* more) {
+                                  const int* before, int* more) {
+  // a round after the one that finished has nothing to do (its input buffer is the result)
+  if (before && *before == 0) return;
   int again = 0;
   for (long long v = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; v < n;
        v += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -343,15 +345,18 @@ int mosp_path_costs(Context& ctx, Graph& g, Mosp& m, int columns) {
   const Tree& t = m.tree();
   const int grid = ctx.sm_count * 8;
   m.first.reserve(static_cast<size_t>(std::max(n, 1LL)));
-  m.missing.reserve(2);  // [0] the lowest vertex without its tree edge, [1] "jump again"
+  // [0] the lowest vertex without its tree edge, [1 + r] "jump again" of round r
+  constexpr int kRounds = 64;
+  m.missing.reserve(1 + kRounds);
   int* more_flag = m.missing.ptr + 1;
   for (int b = 0; b < 2; ++b) {
     m.anc[b].reserve(static_cast<size_t>(std::max(n, 1LL)));
     m.acc[b].reserve(static_cast<size_t>(std::max(n, 1LL)) * columns);
   }
   DYNGB200_CUDA(cudaMemsetAsync(m.first.ptr, 0xff, n * sizeof(unsigned), s));
-  const int big = 0x7fffffff;
-  DYNGB200_CUDA(cudaMemcpyAsync(m.missing.ptr, &big, sizeof(int), cudaMemcpyHostToDevice, s));
+  constexpr int big = 0x7f7f7f7f;  // above every vertex id of a graph that fits the device
+  DYNGB200_CUDA(cudaMemsetAsync(m.missing.ptr, 0x7f, sizeof(int), s));
+  DYNGB200_CUDA(cudaMemsetAsync(more_flag, 0, kRounds * sizeof(int), s));
   const GraphView gv = g.view();
   if (g.props.allow_multi)
     k_mosp_first_scan<<<grid, kMospBlock, 0, s>>>(gv, n, t.parent.ptr, m.source, m.first.ptr);
@@ -362,22 +367,33 @@ int mosp_path_costs(Context& ctx, Graph& g, Mosp& m, int columns) {
                                                 m.missing.ptr);
   ctx.launches += 2;
   DYNGB200_CUDA(cudaGetLastError());
-  int b = 0;
-  for (int round = 0; round < 64; ++round) {
-    DYNGB200_CUDA(cudaMemsetAsync(more_flag, 0, sizeof(int), s));
-    k_mosp_costs_jump<<<grid, kMospBlock, 0, s>>>(n, columns, m.acc[b].ptr, m.anc[b].ptr,
-                                                  m.acc[1 - b].ptr, m.anc[1 - b].ptr, more_flag);
-    ++ctx.launches;
+  // Rounds are queued several at a time, so that the host waits once for all of them (a wait and a
+  // read-back per round were half of the step); the ones past the last that moved a vertex return
+  // at once.  Six rounds sum the paths of trees up to 64 edges deep.
+  int b = 0, missing = big;
+  for (int round = 0; round < kRounds;) {
+    constexpr int kBatch = 6;
+    const int first = round;
+    for (; round < std::min(first + kBatch, kRounds); ++round) {
+      const int in = (b + round - first) & 1;
+      k_mosp_costs_jump<<<grid, kMospBlock, 0, s>>>(n, columns, m.acc[in].ptr, m.anc[in].ptr,
+                                                    m.acc[1 - in].ptr, m.anc[1 - in].ptr,
+                                                    round > first ? more_flag + round - 1 : nullptr,
+                                                    more_flag + round);
+      ++ctx.launches;
+    }
     DYNGB200_CUDA(cudaGetLastError());
-    b = 1 - b;
-    int more = 0;
-    DYNGB200_CUDA(cudaMemcpyAsync(&more, more_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
+    int seen[1 + kRounds];
+    DYNGB200_CUDA(cudaMemcpyAsync(seen, m.missing.ptr, (1 + round) * sizeof(int),
+                                  cudaMemcpyDeviceToHost, s));
     DYNGB200_CUDA(cudaStreamSynchronize(s));
-    if (!more) break;
+    missing = seen[0];
+    int ran = first;  // the rounds that ran: up to and including the first without another jump
+    while (ran < round && seen[1 + ran] != 0) ++ran;
+    const bool done = ran < round;
+    b = (b + (done ? ran + 1 : round) - first) & 1;
+    if (done) break;
   }
-  int missing = big;
-  DYNGB200_CUDA(cudaMemcpyAsync(&missing, m.missing.ptr, sizeof(int), cudaMemcpyDeviceToHost, s));
-  DYNGB200_CUDA(cudaStreamSynchronize(s));
   if (missing != big) {
     int32_t p = -1;
     DYNGB200_CUDA(cudaMemcpy(&p, t.parent.ptr + missing, sizeof(int32_t), cudaMemcpyDeviceToHost));

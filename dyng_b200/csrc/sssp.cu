@@ -286,7 +286,7 @@ struct Offer {
 
 __device__ __forceinline__ void push_prepare(const SsspParams& p, Ctx& X, int u, u64 du, int y,
                                              int w, Offer& r) {
-  ++X.slots;
+  X.slots += y >= kDead;
   r.dst = y;
   r.cand = kPackedInf;
   r.cur = 0;
@@ -428,30 +428,34 @@ __device__ __forceinline__ void warp_rows(const SsspParams& p, Ctx& X, int owner
   const int32_t* col = row_col<MODE>(p);
   const int32_t* wt = row_w<MODE>(p);
   if (MODE == kPush) {
-    // two slots per lane and step: both offers prepared before either commits
+    // two slots per lane and step: both offers prepared before either commits; the slots are loaded
+    // before the owners' distances are looked at
     for (int base = 0; base < total; base += 64) {
-      Offer r[2];
+      int j[2], y[2], w[2];
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
         const int e = base + 32 * q + lane;
-        int j = 0;
+        j[q] = 0;
 #pragma unroll
         for (int step = 16; step > 0; step >>= 1) {
-          const int cand = j + step;
-          if (__shfl_sync(0xffffffffu, excl, cand) <= e) j = cand;
+          const int cand = j[q] + step;
+          if (__shfl_sync(0xffffffffu, excl, cand) <= e) j[q] = cand;
         }
-        const int o = __shfl_sync(0xffffffffu, owner, j);
-        const u64 d = __shfl_sync(0xffffffffu, odu, j);
-        const unsigned s = __shfl_sync(0xffffffffu, start, j);
-        const int ex = __shfl_sync(0xffffffffu, excl, j);
+        const unsigned s = __shfl_sync(0xffffffffu, start, j[q]);
+        const int ex = __shfl_sync(0xffffffffu, excl, j[q]);
+        y[q] = kNoSlot;
+        w[q] = 0;
         if (e < total) {
-          const unsigned slot = s + static_cast<unsigned>(e - ex);
-          push_prepare(p, X, o, d, col[slot], wt[slot], r[q]);
-        } else {
-          r[q].cand = kPackedInf;
-          r[q].cur = 0;
-          r[q].dst = -1;
+          y[q] = col[s + static_cast<unsigned>(e - ex)];
+          w[q] = wt[s + static_cast<unsigned>(e - ex)];
         }
+      }
+      Offer r[2];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int o = __shfl_sync(0xffffffffu, owner, j[q]);
+        const u64 d = __shfl_sync(0xffffffffu, odu, j[q]);
+        push_prepare(p, X, o, d, y[q], w[q], r[q]);
       }
       push_commit<2>(p, X, r);
     }

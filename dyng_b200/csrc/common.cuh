@@ -13,7 +13,7 @@ constexpr int64_t kInfinity = INT64_MAX / 4;  // sssp_infinity of the reference 
 constexpr u64 kPackedInf = ~0ULL;
 constexpr int32_t kDead = -1;  // tombstone in a slack row's column slot
 constexpr long long kDenseDegree = 6;  // edges per vertex from which paths and trees are taken as short
-constexpr int kDefaultSmall = 256;  // the heuristic: frontiers up to 256 vertices run on one block
+constexpr int kDefaultSmall = 256;  // the heuristic's small-frontier size (dyngb200_schedule)
 
 // Device error bits (the sticky error word; the reference's util/device_error_flags.hpp:9-43
 // has capacity / invalid_input / parent_cycle / internal).

@@ -5,13 +5,18 @@
 //
 // What differs from the reference's kernel (the results do not):
 //   - the packed (distance << b | parent) words persist between updates in the tree, so an update
-//     does not pack all n vertices; the unpack compares every word with its (distance, parent)
-//     and writes the changed ones (`affected`), so the relaxations keep no list of written words;
-//   - frontier rows longer than `heavy_degree` are split into 1024-slot chunks spread over all
-//     warps (one 64-bit atomic reserves a list slot and its chunk range together), shorter rows
-//     of 32+ slots are scanned by a whole warp, the rest by one lane each;
-//   - the grid barrier is this file's own, with a time limit after which it records kErrTimeout
+//     does not pack all n vertices; the commit compares the words that this call changed with their
+//     (distance, parent) and writes the changed ones (`affected`);
+//   - frontier rows longer than `heavy_degree` are split into kHeavyChunk-slot chunks spread over
+//     all warps (one 64-bit atomic reserves a list slot and its chunk range together), rows of more
+//     than kLightMax slots are scanned by a whole warp, the rest share a warp;
+//   - a short frontier of light rows stays with the blocks that found it, round after round;
+//   - the grid barrier is this library's own, with a time limit after which it records kErrTimeout
 //     and every block leaves the kernel (no unbounded spin).
+//
+// The kernel is bound by latency, not bandwidth: dependent loads (list entry, row, neighbour's
+// word) and the barriers between steps whose frontiers shrink geometrically; see the comments at
+// the steps for what each costs.
 #include "internal.hpp"
 #include "grid_sync.cuh"
 #include "sssp_params.cuh"

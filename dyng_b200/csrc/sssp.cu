@@ -813,7 +813,7 @@ __device__ __forceinline__ void clear_step(UpdateCtl* c, int it) {
 
 // The invalidation without a schedule's say: a top-down walk of the invalidated subtrees where
 // the changed tree edges are few, pointer jumping otherwise.  Pointer jumping visits every vertex
-// in each of its four to seven rounds (100 us at 4.2M vertices, 29 us at a thousand); the walk
+// in each of its four to seven rounds (85 us at 4.2M vertices, 20 us at a thousand); the walk
 // reads the out-rows of the invalidated vertices alone, but takes as many levels as their subtrees
 // are deep.  So it is tried on graphs of at least kDenseDegree edges per vertex (shallow trees; on
 // a grid the subtrees are thousands of levels deep) with few roots, and what is not reached after
@@ -824,6 +824,13 @@ constexpr long long kWalkRoots = 32;      // or one per kWalkShare vertices wher
 constexpr long long kWalkShare = 16384;
 constexpr long long kWalkLarge = 1 << 20;  // six levels from here on, two below
 constexpr int kWalkPairs = 2048;  // larger batches hardly hold so few roots: not listed for it
+
+// Pointer jumping starts from a sequential pass that lays out every vertex's ancestor, except on
+// graphs of at most kPjShort vertices, whose first round reads the stamps and parents itself: a
+// barrier less, two random words per gather instead of one.  Invalidation with 4 rounds, the pass
+// and one hop per round before, now: 41 -> 31 us at 262,144 vertices / 10k changes, 28 -> 16 at
+// 12,345 / 601; at 1,048,576 vertices leaving the pass out measured 60 us, keeping it 56.
+constexpr long long kPjShort = 1LL << 18;
 
 // A block's own levels of the walk: the subtrees below the vertices that it invalidated (a vertex
 // has one tree parent, so no two blocks meet).  What does not fit is shared with the grid.
@@ -1198,6 +1205,11 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
         // ancestor) entries per block) with no global atomic.  Later rounds see the regions, concatenated in block
         // order, as one list (each block scans the per-block counts) and split it evenly over
         // the blocks: a block visits at most `span` entries, so its survivors fit its region.
+        // A later round has few entries and is bound by its barrier and round trips, so it goes
+        // kPjHops ancestors on instead of one (any ancestor that it reads is a valid one): 4
+        // rounds become 3 at R-MAT scale 22 / 100k changes (117 -> 104 us), 7 become 4 on a
+        // 1,000 x 1,000 grid (129 -> 84 us).  Round 0, bound by its gathers, jumps once (twice
+        // without the pass).
         __shared__ int s_pj_cnt;
         __shared__ int s_prefix[kPjMaxBlocks + 1];
         const long long span = (n + nblk - 1) / nblk;
@@ -1215,7 +1227,10 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
         // about a quarter of the bandwidth); the tail, and unaligned arrays, word by word
         const bool vec = ((reinterpret_cast<uintptr_t>(p.stamp) | reinterpret_cast<uintptr_t>(p.parent) |
                            reinterpret_cast<uintptr_t>(p.ancestor)) & 15) == 0;
-        const long long quads = vec ? min(n, p.tree_n) >> 2 : 0;
+        // On small graphs a round is bound by its barrier and round trips, not by the gathers: the
+        // first round reads stamps and parents itself instead of waiting for this pass.
+        const bool short_rounds = n <= kPjShort;
+        const long long quads = vec && !short_rounds ? min(n, p.tree_n) >> 2 : 0;
         for (long long q0 = tid; q0 < quads; q0 += 2 * threads) {
           int4 st[2], pa[2];
 #pragma unroll
@@ -1235,51 +1250,31 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
                             first_ancestor(st[j].z, pa[j].z), first_ancestor(st[j].w, pa[j].w));
           }
         }
-        for (long long v = 4 * quads + tid; v < n; v += threads)
-          p.ancestor[v] = first_ancestor(ld_cg(&p.stamp[v]), v < p.tree_n ? p.parent[v] : -1);
-        if (tid == 0) c->work[22] = n;
-        if (!grid_barrier(c, bar)) return;
+        if (!short_rounds) {
+          for (long long v = 4 * quads + tid; v < n; v += threads)
+            p.ancestor[v] = first_ancestor(ld_cg(&p.stamp[v]), v < p.tree_n ? p.parent[v] : -1);
+          if (tid == 0) c->work[22] = n;
+          if (!grid_barrier(c, bar)) return;
+        }
+        // an ancestor before the first short round has written any
+        auto tree_ancestor = [&](int v) {
+          return first_ancestor(ld_cg(&p.stamp[v]), v < p.tree_n ? p.parent[v] : -1);
+        };
+        constexpr int kPjHops = 3;
+        long long total = n;
         for (int round = 0; round < max_rounds; ++round) {
           if (tid == 0) {
             c->rounds = round + 1;
             if (round < 24) c->pj_t[round] = static_cast<unsigned>(global_ns() - c->phase_ns[0]);
           }
           if (threadIdx.x == 0) s_pj_cnt = 0;
-          long long total = n;
-          if (round > 0) {
-            const int* cnt = p.pj_blk + ((round - 1) & 1) * kPjMaxBlocks;
-            for (int q = threadIdx.x; q < nblk; q += blockDim.x) s_prefix[q + 1] = ld_cg(&cnt[q]);
-            if (threadIdx.x == 0) s_prefix[0] = 0;
-            __syncthreads();
-            if (threadIdx.x < 32) {
-              // inclusive scan of s_prefix[1..nblk] by warp 0: chunks of `per`, then the chunk sums
-              const int per = (nblk + 31) / 32;
-              const int b0 = 1 + lane * per, b1 = min(nblk + 1, b0 + per);
-              int run = 0;
-              for (int q = b0; q < b1; ++q) {
-                run += s_prefix[q];
-                s_prefix[q] = run;
-              }
-              int incl = run;
-              for (int o = 1; o < 32; o <<= 1) {
-                const int t = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += t;
-              }
-              const int before = incl - run;
-              for (int q = b0; q < b1; ++q) s_prefix[q] += before;
-            }
-            __syncthreads();
-            total = s_prefix[nblk];
-          } else {
-            __syncthreads();
-          }
+          __syncthreads();
           const long long vspan = (total + nblk - 1) / nblk;
           const long long vlo = static_cast<long long>(blockIdx.x) * vspan;
           const long long vhi = min(total, vlo + vspan);
           // survivor entries are (vertex, its ancestor): a round gathers only ancestor[a]
           const int2* cur = (round & 1) ? p.heavy_a : p.heavy_b;  // the previous round's regions
           int2* next = ((round & 1) ? p.heavy_b : p.heavy_a) + lo;  // this block's region
-          int jumping = 0;
           // four entries per thread and step, their loads issued together; the warps iterate
           // together (the bound is tested on the warp's first entry) for the ballots below
           for (long long i0 = vlo + (threadIdx.x & ~31); i0 < vhi; i0 += 4LL * blockDim.x) {
@@ -1305,14 +1300,37 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
                 a[q] = e.y;
               }
             }
-            if (round == 0) {
+            if (round == 0 && short_rounds) {
 #pragma unroll
-              for (int q = 0; q < 4; ++q) a[q] = vv[q] < 0 ? -1 : ld_cg(&p.ancestor[vv[q]]);
-            }
+              for (int q = 0; q < 4; ++q) a[q] = vv[q] < 0 ? -1 : tree_ancestor(vv[q]);
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              na[q] = a[q] < 0 ? a[q] : ld_cg(&p.ancestor[a[q]]);
-              if (na[q] == p.source) na[q] = -1;  // reaching the source ends a chain
+              for (int q = 0; q < 4; ++q) {
+                w_jumps += a[q] >= 0;
+                na[q] = a[q] < 0 ? a[q] : tree_ancestor(a[q]);
+              }
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                if (na[q] < 0) continue;
+                ++w_jumps;
+                na[q] = tree_ancestor(na[q]);
+              }
+            } else {
+              if (round == 0) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) a[q] = vv[q] < 0 ? -1 : ld_cg(&p.ancestor[vv[q]]);
+              }
+#pragma unroll
+              for (int q = 0; q < 4; ++q) na[q] = a[q];
+              const int hops = round == 0 ? 1 : kPjHops;
+              for (int hop = 0; hop < hops; ++hop) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                  if (na[q] < 0) continue;
+                  ++w_jumps;
+                  na[q] = ld_cg(&p.ancestor[na[q]]);
+                  if (na[q] == p.source) na[q] = -1;  // reaching the source ends a chain
+                }
+              }
             }
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -1321,7 +1339,6 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
               if (v >= 0) {
                 ++w_visits;
                 if (a[q] >= 0) {
-                  ++w_jumps;
                   if (na[q] == kMarked) {
                     p.ancestor[v] = kMarked;
                     p.stamp[v] = gen_inv;
@@ -1331,6 +1348,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
                     p.ancestor[v] = na[q];
                     survives = na[q] >= 0;
                   }
+                } else if (round == 0 && short_rounds) {
+                  p.ancestor[v] = a[q];
                 }
               }
               // warp-aggregated append to the block's survivor region
@@ -1340,25 +1359,43 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
                 if (lane == 0) base = atomicAdd(&s_pj_cnt, __popc(m));
                 base = __shfl_sync(0xffffffffu, base, 0);
                 if (survives) next[base + __popc(m & ((1u << lane) - 1))] = make_int2(v, na[q]);
-                jumping = 1;
               }
             }
           }
           __syncthreads();
           if (threadIdx.x == 0) p.pj_blk[(round & 1) * kPjMaxBlocks + blockIdx.x] = s_pj_cnt;
-          (void)jumping;
           if (!grid_barrier(c, bar)) return;
           if (tid == 0 && round < 24)
             c->pj_done[round] = static_cast<unsigned>(global_ns() - c->phase_ns[0]);
-          // every block reads the survivor counts itself: none left, the rounds are done (no
-          // flag that every warp with a survivor would store)
+          // every block scans the survivor counts itself: none left, the rounds are done (no flag
+          // that every warp with a survivor would store); else their prefix sums lay out the next
+          // round's entries
           {
             const int* cnt = p.pj_blk + (round & 1) * kPjMaxBlocks;
-            int mine = 0;
-            for (int q = threadIdx.x; q < nblk; q += blockDim.x) mine |= ld_cg(&cnt[q]);
-            const int any = __syncthreads_or(mine != 0);
-            if (tid == 0) c->active[round % 3] = any;  // the host's parent-cycle check
-            if (!any) break;
+            for (int q = threadIdx.x; q < nblk; q += blockDim.x) s_prefix[q + 1] = ld_cg(&cnt[q]);
+            if (threadIdx.x == 0) s_prefix[0] = 0;
+            __syncthreads();
+            if (threadIdx.x < 32) {
+              // inclusive scan of s_prefix[1..nblk] by warp 0: chunks of `per`, then the chunk sums
+              const int per = (nblk + 31) / 32;
+              const int b0 = 1 + lane * per, b1 = min(nblk + 1, b0 + per);
+              int run = 0;
+              for (int q = b0; q < b1; ++q) {
+                run += s_prefix[q];
+                s_prefix[q] = run;
+              }
+              int incl = run;
+              for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += t;
+              }
+              const int before = incl - run;
+              for (int q = b0; q < b1; ++q) s_prefix[q] += before;
+            }
+            __syncthreads();
+            total = s_prefix[nblk];
+            if (tid == 0) c->active[round % 3] = total != 0;  // the host's parent-cycle check
+            if (total == 0) break;
           }
         }
       }

@@ -6,7 +6,8 @@ against the oracle bit for bit:
   - threshold raises that find nothing below the new threshold and skip to the next distance;
   - relocated rows around the length above which a row moves in chunks;
   - host batches around the size that comes over with the control block;
-  - the subtree walk that an update without a schedule tries when few tree edges changed.
+  - the subtree walk that an update without a schedule tries when few tree edges changed;
+  - pointer jumping on either side of the size up to which it starts without a seeding pass.
 """
 import numpy as np
 import pytest
@@ -18,6 +19,7 @@ from tests.helpers import random_batch
 pytestmark = pytest.mark.gpu
 
 MOVE_CHUNK = 512          # slots of a row that move as one piece
+PJ_SHORT = 1 << 18        # vertices up to which pointer jumping starts from the tree itself
 STAGED_VALUES = 64 * 1024 // 4  # values of a host batch that come over with the control block
 
 
@@ -208,3 +210,23 @@ def test_few_changed_tree_edges(roots, depth):
     back = dict(ins_src=b["del_src"], ins_dst=b["del_dst"], ins_w=np.full(roots, 3, np.int32),
                 del_src=empty, del_dst=empty)
     _update(g, og, t, ot, back, "mend")
+
+
+@pytest.mark.parametrize("depth", [1, 2, 3, 4, 40, 3000])
+@pytest.mark.parametrize("n", [PJ_SHORT - 1, PJ_SHORT, PJ_SHORT + 1, PJ_SHORT + 5])
+def test_pointer_jumping_around_the_seeded_size(n, depth):
+    # chains of `depth` below the source (sparse: no walk), cut at random places, the last vertex
+    # among them; every vertex keeps a heavy edge from the source
+    rng = np.random.default_rng(n + depth)
+    v = np.arange(1, n)
+    src = np.concatenate([np.where((v - 1) % depth == 0, 0, v - 1), np.zeros(n - 1)])
+    dst = np.concatenate([v, v])
+    w = np.concatenate([rng.integers(1, 9, n - 1), np.full(n - 1, 10 * depth)])
+    keep = (src[: n - 1] != 0).tolist() + [True] * (n - 1)  # one edge from the source per vertex
+    src, dst, w = _i32(src[keep], dst[keep], w[keep])
+    g, og, t, ot = _both(n, src, dst, w)
+    cut = np.append(rng.choice(np.arange(1, n - 1), 60, replace=False), n - 1).astype(np.int32)
+    empty = cut[:0]
+    b = dict(ins_src=empty, ins_dst=empty, ins_w=empty, del_src=ot.parents[cut], del_dst=cut)
+    st = _update(g, og, t, ot, b, "cut")
+    assert st.invalidation == 0 and (depth < 3 or st.invalidated >= cut.size)

@@ -1319,16 +1319,19 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
 #pragma unroll
                 for (int q = 0; q < 4; ++q) a[q] = vv[q] < 0 ? -1 : ld_cg(&p.ancestor[vv[q]]);
               }
+              // the loads of a hop are selected, not branched over: the four go out together
 #pragma unroll
-              for (int q = 0; q < 4; ++q) na[q] = a[q];
-              const int hops = round == 0 ? 1 : kPjHops;
-              for (int hop = 0; hop < hops; ++hop) {
+              for (int q = 0; q < 4; ++q) {
+                w_jumps += a[q] >= 0;
+                na[q] = a[q] < 0 ? a[q] : ld_cg(&p.ancestor[a[q]]);
+                if (na[q] == p.source) na[q] = -1;  // reaching the source ends a chain
+              }
+              for (int hop = 1; hop < kPjHops && round > 0; ++hop) {
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                  if (na[q] < 0) continue;
-                  ++w_jumps;
-                  na[q] = ld_cg(&p.ancestor[na[q]]);
-                  if (na[q] == p.source) na[q] = -1;  // reaching the source ends a chain
+                  w_jumps += na[q] >= 0;
+                  na[q] = na[q] < 0 ? na[q] : ld_cg(&p.ancestor[na[q]]);
+                  if (na[q] == p.source) na[q] = -1;
                 }
               }
             }

@@ -1822,10 +1822,12 @@ void Workspace::reserve_vertices(long long n_cap, cudaStream_t s) {
     b->release();
     b->reserve(n, s);
   }
-  for (DevBuf<int>* b : {&heavy_a, &heavy_b, &pull_heavy}) {  // int2 entries
+  for (DevBuf<int>* b : {&heavy_a, &heavy_b}) {  // int2 entries
     b->release();
-    b->reserve(2 * n, s);
+    b->reserve(2 * static_cast<size_t>(pj_list_entries(n_cap)), s);
   }
+  pull_heavy.release();
+  pull_heavy.reserve(2 * n, s);  // int2 entries
   generation = 0;
   touch_generation = 0;
   n_sized = n_cap;

@@ -200,6 +200,9 @@ struct UpdateCtl {
 
 // Persistent blocks the pointer-jumping survivor lists of the sssp kernel support.
 constexpr int kPjMaxBlocks = 1024;
+// Entries of such a list (heavy_a, heavy_b) for n_cap vertices.  Block b of B writes its survivors
+// from b * ceil(n / B) on: the regions end up to B - 1 entries past n.
+constexpr long long pj_list_entries(long long n_cap) { return n_cap + kPjMaxBlocks; }
 
 // Stamp generations: a claim of the near-far loop holds a generation and a block in one int.
 constexpr int kClaimBlockBits = 10;

@@ -1204,7 +1204,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
         // again) is written to its block's survivor region (heavy_a / heavy_b, `span` (vertex,
         // ancestor) entries per block) with no global atomic.  Later rounds see the regions, concatenated in block
         // order, as one list (each block scans the per-block counts) and split it evenly over
-        // the blocks: a block visits at most `span` entries, so its survivors fit its region.
+        // the blocks: a block visits at most `span` entries, so its survivors fit its region (the
+        // last regions reach past n: pj_list_entries).
         // A later round has few entries and is bound by its barrier and round trips, so it goes
         // kPjHops ancestors on instead of one (any ancestor that it reads is a valid one): 4
         // rounds become 3 at R-MAT scale 22 / 100k changes (117 -> 104 us), 7 become 4 on a

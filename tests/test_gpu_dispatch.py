@@ -7,7 +7,8 @@ against the oracle bit for bit:
   - relocated rows around the length above which a row moves in chunks;
   - host batches around the size that comes over with the control block;
   - the subtree walk that an update without a schedule tries when few tree edges changed;
-  - pointer jumping on either side of the size up to which it starts without a seeding pass.
+  - pointer jumping on either side of the size up to which it starts without a seeding pass, and
+    on a graph that fills its vertex capacity.
 """
 import numpy as np
 import pytest
@@ -230,3 +231,32 @@ def test_pointer_jumping_around_the_seeded_size(n, depth):
     b = dict(ins_src=empty, ins_dst=empty, ins_w=empty, del_src=ot.parents[cut], del_dst=cut)
     st = _update(g, og, t, ot, b, "cut")
     assert st.invalidation == 0 and (depth < 3 or st.invalidated >= cut.size)
+
+
+@pytest.mark.parametrize("blocks", [444, 300, 7, 0])
+def test_pointer_jumping_of_a_graph_at_its_vertex_capacity(blocks):
+    # 1,000 vertices leave room for 1,024 + 62 more; one batch brings them all.  A chain of `length`
+    # leaves about as many survivors after round 0: 1,720 deal four entries a block where the
+    # regions are five apart, so the last regions lie past the last vertex
+    for length in (1723, 1600, 900, 2080):
+        n0, n = 1000, 2086
+        v = np.arange(1, n)
+        parent = np.where((v > 1) & (v <= length), v - 1, 0)
+        w = np.full(n - 1, 2)
+        old = v < n0
+        src, dst, w = _i32(parent, v, w)
+        res = D.Resources()
+        g = D.Graph.from_edges(src[old], dst[old], w[old], n0, resources=res)
+        og = O.Graph.from_edges(n0, src[old], dst[old], w[old], 1)
+        t = D.sssp.compute(g, 0)
+        ot, _ = O.compute(og, 0, rule=1)
+        empty = src[:0]
+        grow = dict(ins_src=src[~old], ins_dst=dst[~old], ins_w=w[~old], del_src=empty, del_dst=empty)
+        _update(g, og, t, ot, grow, "grow")
+        cut = np.asarray([length - 3, length // 2, n - 1])
+        b = dict(ins_src=empty, ins_dst=empty, ins_w=empty, del_src=parent[cut - 1].astype(np.int32),
+                 del_dst=cut.astype(np.int32))
+        _update(g, og, t, ot, b, "cut", D.sssp.Schedule(grid_blocks=blocks))
+        back = dict(ins_src=b["del_src"], ins_dst=b["del_dst"], ins_w=np.full(cut.size, 3, np.int32),
+                    del_src=empty, del_dst=empty)
+        _update(g, og, t, ot, back, "mend", D.sssp.Schedule(grid_blocks=blocks))

@@ -1053,7 +1053,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
   X.low = kPackedInf;
   X.slots = X.words = X.atomics = X.appends = X.rows = X.tries = 0;
   const Packing pk = X.pk;
-  const u64 delta = static_cast<u64>(p.delta_override > 0 ? p.delta_override : c->delta * p.width_scale);
+  const u64 delta = static_cast<u64>(p.delta_override > 0 ? p.delta_override : c->delta);
   int gen = p.generation;
   // work counters (see dyngb200_stats::work)
   long long w_visits = 0, w_jumps = 0, w_inval = 0;
@@ -1740,22 +1740,12 @@ static void launch(Context& ctx, SsspParams& p, int blocks) {
                                             dim3(kThreads), args, 0, ctx.stream));
 }
 
-// Raises of the threshold by the automatic width (32 x average weight / average degree) times this.
-// Graphs of several edges per vertex are a few hops wide, so a wider bucket saves whole steps for
-// few pushes done twice; on sparse ones it pushes long wrong paths.  Passes with 1, 2, 4 and 8
-// times the width: R-MAT scale 18 / 10k changes 719, 696, 684, 684 us, scale 22 / 1k 812, 772, 772,
-// 777, scale 20 deletions 1,447, 1,409, 1,390, 1,388; 1000^2 grid churn 2,655, 2,877, 3,402, 3,475.
-static int auto_width_scale(const Graph& g, long long delta_opt) {
-  return delta_opt > 0 || g.m < kDenseDegree * g.n ? 1 : 4;
-}
-
 static SsspParams base_params(Context& ctx, Graph& g, Tree& t) {
   Workspace& ws = ctx.ws;
   SsspParams p{};
   p.g = g.view();
   p.objective = t.opt.objective;
   p.source = t.source;
-  p.width_scale = auto_width_scale(g, t.opt.delta);
   p.dist = reinterpret_cast<long long*>(t.dist.ptr);
   p.parent = t.parent.ptr;
   p.packed = t.packed.ptr;
@@ -2428,7 +2418,6 @@ void sssp_compute_static(Graph& g, int32_t source, int objective, long long delt
   p.touch_gen = 1;
   p.heavy_degree = 256;
   p.small_frontier = kDefaultSmall;
-  p.width_scale = auto_width_scale(g, delta);
   u64 bound = 0;
   const Packing pk = choose_packing(n, cs.max_w, &bound);
   p.tree_bits = pk.bits;

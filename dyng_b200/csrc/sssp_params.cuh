@@ -50,7 +50,6 @@ struct SsspParams {
   int touch_gen;
   int heavy_degree;
   long long delta_override;
-  int width_scale;       // a raise of the threshold is the plan's width times this
   int small_frontier;    // short near frontiers stay with the blocks that found them (0: never)
   UpdateCtl* ctl;
   TreeHistory* hist;

@@ -111,8 +111,7 @@ typedef struct dyngb200_stats {
   int64_t pushes;      /* schedule-dependent */
   int32_t packed_parents;
   int32_t engine_used; /* dyngb200_engine that ran: FUSED or OPERATORS */
-  int64_t delta;       /* near-far width of the plan or schedule (a raise by an automatic width
-                        * covers four of it on graphs of six or more edges per vertex) */
+  int64_t delta;       /* near-far width that ran */
   int64_t max_weight;  /* bound weight of the packing */
   int32_t grid_blocks; /* persistent grid that ran (operators engine: its launches' grid) */
   int32_t invalidation; /* 0 pointer jumping, 1 subtree walk */

@@ -169,6 +169,30 @@ def test_learned_updates_equal_plain_updates(D):
     assert len(seen) >= 3
 
 
+def test_the_default_classes_are_the_plain_schedule(D):
+    # a uniform graph whose whole tree hangs on one edge: the repair after the cut pushes 1.7 times
+    # as many vertices with another width (runs of one width differ by a few percent)
+    from dyng_b200 import scheduler as S
+    rng = np.random.default_rng(9)
+    n = 200_000
+    s, d = rng.integers(1, n, (2, 8 * n)).astype(np.int32)
+    s, d = np.append(s, [0, 0]).astype(np.int32), np.append(d, [1, 2]).astype(np.int32)
+    w = np.append(rng.integers(1, 1000, 8 * n), [1, 10**6]).astype(np.int32)
+    g = D.Graph.from_edges(s, d, w, num_vertices=n)
+    tree = D.sssp.compute(g, 0)
+    cut = D.EdgeBatch.from_arrays([], [], [], [0], [1])
+    back = D.EdgeBatch.from_arrays([0], [1], [1], [], [])
+    plain = [D.sssp.update(g, b, tree) for b in (cut, back)]
+    want = [t.copy() for t in (tree.distances, tree.parents)]
+    named = S.schedule_for(S.DEFAULT_CLASSES, plain[0].delta, plain[0].grid_blocks)
+    again = [D.sssp.update(g, b, tree, schedule=named) for b in (cut, back)]
+    for st, other in zip(plain, again):
+        assert (st.delta, st.grid_blocks, st.invalidation, st.epochs) == \
+            (other.delta, other.grid_blocks, other.invalidation, other.epochs)
+        assert abs(st.pushes - other.pushes) < 0.25 * other.pushes
+    assert np.array_equal(tree.distances, want[0]) and np.array_equal(tree.parents, want[1])
+
+
 def test_outside_its_trained_range_the_scheduler_keeps_the_plain_schedule(D):
     from dyng_b200 import scheduler as S
     rng = np.random.default_rng(12)

@@ -706,9 +706,13 @@ struct LoopState {
 // Inside one bucket the order of the pushes does not matter for the result (every push is an
 // atomicMin), so no other block has to wait for them; a step of the grid is bound by its barriers
 // and list round trips (8-10 us for a few hundred vertices, 3-4 us for a block's round).  Only
-// frontiers of light rows run this way, up to kLocalShare x the schedule's small-frontier size:
-// longer ones keep every warp busy, and the blocks would push a vertex once for every block
-// that reached it (a 24k-vertex R-MAT frontier measured 1.6x slower).
+// frontiers of light rows run this way, up to the schedule's small-frontier size, or kLocalShare
+// times it on graphs below kDenseDegree edges per vertex.  A frontier of a dense graph grows several
+// times over in a round: its blocks fill up at different times, most of them wait for the one with
+// the most rounds, and vertices are pushed once for every block that reached them.  Near-far of the
+// repair after a cut near the source, with limits of none, 256 and 16,384 vertices: uniform 20,000 x
+// 8 edges 214, 228, 308 us, 60,000 x 8 250, 225, 338, 200,000 x 8 329, 322, 410, 200,000 x 4 340, 291,
+// 268; of 2 % random changes at 200,000 x 4 217, 181, 154; grid 500^2 912, 587, 341.
 constexpr int kLocalLight = 128;    // stage entries a block keeps (more: the grid shares them)
 constexpr int kLocalMed = 8;
 constexpr int kLocalRounds = 1024;  // rounds before the block meets the others again
@@ -889,6 +893,8 @@ __device__ bool near_far(const SsspParams& p, Ctx& X, LoopState& S, unsigned& ba
   int* mlists[2] = {p.near_med_a, p.near_med_b};
   int2* hlists[2] = {p.heavy_a, p.heavy_b};
   const Packing pk = X.pk;
+  const long long local_max =
+      small * (p.g.counters->m < kDenseDegree * n ? static_cast<long long>(kLocalShare) : 1LL);
   while (true) {
     const int cs = S.it % 3;
     const int nc = ld_cg(&c->near_cnt[cs]);
@@ -923,8 +929,7 @@ __device__ bool near_far(const SsspParams& p, Ctx& X, LoopState& S, unsigned& ba
       }
       ++S.iterations;
       ++S.gen;
-      const bool local = small > 0 && hc == 0 && mc == 0 &&
-                         nc <= kLocalShare * static_cast<long long>(small);
+      const bool local = hc == 0 && mc == 0 && nc <= local_max;
       X.gen = near_claim(S.gen, local ? static_cast<int>(blockIdx.x) : kClaimGrid);
       const int nb = (S.it + 1) & 1;
       X.next = ListSet{lists[nb], &c->near_cnt[(S.it + 1) % 3], mlists[nb],

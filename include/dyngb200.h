@@ -176,8 +176,9 @@ typedef struct dyngb200_schedule {
   int32_t grid_blocks;    /* persistent grid size (0: occupancy x SMs, fewer on small graphs) */
   int32_t invalidation;   /* 0 heuristic: pointer jumping, or the subtree walk where few tree edges
                            * of a dense graph changed; 1 subtree walk */
-  int32_t small_frontier; /* near frontiers of at most 64 x this many light rows stay with the blocks
-                           * that found them for several rounds (0: 256, < 0: off) */
+  int32_t small_frontier; /* near frontiers of at most this many light rows (64 x as many on graphs
+                           * of less than six edges per vertex) stay with the blocks that found
+                           * them for several rounds (0: 256, < 0: off) */
   int32_t heavy_degree;   /* rows longer than this are split across warps (0: default) */
   int32_t record_features; /* nonzero: compute the scheduler's features into the stats */
 } dyngb200_schedule;

@@ -2566,7 +2566,7 @@ static int apply_blocks_per_sm(Context& ctx) {
 // schedule into the control block.
 void apply_launch(Context& ctx, Graph& g, const StagedBatch& b, int objective, long long delta_opt,
                   const dyngb200_schedule* sched, Tree* tree, const Scheduler* learned,
-                  bool stepped) {
+                  bool stepped, int sssp_blocks) {
   if (!stepped) require_cooperative(ctx);
   Workspace& ws = ctx.ws;
   cudaStream_t s = ctx.stream;
@@ -2618,7 +2618,7 @@ void apply_launch(Context& ctx, Graph& g, const StagedBatch& b, int objective, l
     p.feat_parent = tree->parent.ptr;
     p.feat_tree_n = tree->n;
     L.infer_on = 1;
-    learned_infer_args(ctx, *tree, learned, &L.infer);
+    learned_infer_args(*tree, learned, sssp_blocks, &L.infer);
   }
   L.barrier_limit_ns = ctx.test_barrier_timeout_ns > 0
                            ? static_cast<unsigned long long>(ctx.test_barrier_timeout_ns)

@@ -432,7 +432,8 @@ void scheduler_train(Context& ctx, Scheduler& s, const float* x, const int32_t* 
 // What the batch applier's first block needs to compute the batch features (and, with a
 // scheduler, its schedule) into the control block (mlp_common.cuh)
 struct InferArgs;
-void learned_infer_args(Context& ctx, Tree& t, const Scheduler* sch, InferArgs* out);
+// `blocks`: the grid of the update's sssp launch, which the grid classes scale.
+void learned_infer_args(Tree& t, const Scheduler* sch, int blocks, InferArgs* out);
 
 // The pinned read-back area of a graph: the counters first, then the column statistics.
 constexpr size_t kCounterSlots = (sizeof(GraphCounters) + sizeof(ColumnStats) - 1) / sizeof(ColumnStats);
@@ -464,7 +465,7 @@ struct StagedBatch {
 };
 void apply_launch(Context& ctx, Graph& g, const StagedBatch& b, int objective,
                   long long delta_opt, const dyngb200_schedule* sched, Tree* tree = nullptr,
-                  const Scheduler* learned = nullptr, bool stepped = false);
+                  const Scheduler* learned = nullptr, bool stepped = false, int sssp_blocks = 0);
 void schedule_into(const dyngb200_schedule& sched, UpdateCtl& init);
 // `defer`: a small host batch may come over with the next upload_control instead of now.
 StagedBatch stage_batch(Context& ctx, const dyngb200_batch& batch, int k, bool defer);
@@ -488,7 +489,7 @@ struct PendingUpdate {
   dyngb200_schedule sched{};
   const Scheduler* learned = nullptr;
   StagedBatch b{};
-  int blocks = 0;
+  int blocks = 0;          // of the sssp kernel's launch
   bool operators = false;  // the operators engine (ordinary launches, the loop on the host)
   long long launches0 = 0;
   cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr;  // the context's update events
@@ -506,11 +507,14 @@ void sssp_update_end(PendingUpdate& u, dyngb200_stats* st);
 // (occupancy x SMs, or Context::max_update_blocks when smaller).
 int update_blocks_per_sm(Context& ctx);
 int update_grid_blocks(Context& ctx);
-// The blocks of an sssp launch on a graph of n vertices: a barrier of the whole grid costs 2.2 us,
-// one of a few blocks 1.2, and a small graph keeps no more than a block per 384 vertices busy
-// (measured, sssp kernel of an update: 1,024 vertices 54 us with 444 blocks, 49 with 4; 12,345
-// vertices 113 us, 101 with 32; 65,536 vertices 127 us, 119 with 148; no gain from 260,000 on).
-int update_blocks_for(Context& ctx, long long n);
+// The blocks of an sssp launch on a graph of n vertices and m edges.  A barrier of the whole grid
+// costs 2.2 us, one of a few blocks 1.2, and a small graph keeps no more than a block per 384
+// vertices busy (sssp kernel of an update: 1,024 vertices 54 us with 444 blocks, 49 with 4; 12,345
+// vertices 113 us, 101 with 32; 65,536 vertices 127 us, 119 with 148; no gain from 260,000 on), or
+// one per 4,096 edges where those are more (the repair of a cut tree, uniform 1,024 x 256: 400 us
+// with the 4 blocks of its vertices, 200 with 64, 205 with 444; 4,096 x 512: 1,025 with 11, 280 with
+// 444; 16,384 x 256: 900 with 43, 378 with 444).  A solve pushes every edge: one per 2,048.
+int update_blocks_for(Context& ctx, long long n, long long m, bool from_scratch);
 void sssp_update_each(Context& ctx, Graph& g, const dyngb200_batch& batch, Tree* const* trees,
                       int count, dyngb200_stats* stats);
 void graph_apply(Context& ctx, Graph& g, const dyngb200_batch& batch,

@@ -407,13 +407,13 @@ void scheduler_train(Context& ctx, Scheduler& s, const float* x, const int32_t* 
 // Queued by the applier after its plan (its validation pass accumulated the batch features in
 // the control block): the features and, with a scheduler, the schedule the MLP picks, written
 // into the control block that the persistent kernel reads.
-void learned_infer_args(Context& ctx, Tree& t, const Scheduler* sch, InferArgs* out) {
+void learned_infer_args(Tree& t, const Scheduler* sch, int blocks, InferArgs* out) {
   InferArgs a{};
   a.params = sch ? sch->params.ptr : nullptr;
   a.w = sch ? sch->wbf16.ptr : nullptr;
   if (sch) a.nrm = norm_of(*sch);
   a.hist = t.hist.ptr;
-  a.blocks = update_blocks_for(ctx, t.n);
+  a.blocks = blocks;
   *out = a;
 }
 

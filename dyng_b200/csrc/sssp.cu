@@ -1700,15 +1700,19 @@ void schedule_into(const dyngb200_schedule& sched, UpdateCtl& init) {
   init.active_blocks = sched.grid_blocks > 0 ? sched.grid_blocks : 0;
 }
 
-int update_blocks_for(Context& ctx, long long n) {
-  constexpr long long kVertices = 384;
-  return static_cast<int>(std::min<long long>(update_grid_blocks(ctx),
-                                              std::max(4LL, (n + kVertices - 1) / kVertices)));
+int update_blocks_for(Context& ctx, long long n, long long m, bool from_scratch) {
+  constexpr long long kVertices = 384, kEdges = 4096, kSolveEdges = 2048;
+  const long long edges = from_scratch ? kSolveEdges : kEdges;
+  return static_cast<int>(std::min<long long>(
+      update_grid_blocks(ctx),
+      std::max({4LL, (n + kVertices - 1) / kVertices, (m + edges - 1) / edges})));
 }
 
-static int persistent_blocks(Context& ctx, const dyngb200_schedule& sched, long long n) {
+static int persistent_blocks(Context& ctx, const dyngb200_schedule& sched, long long n, long long m,
+                             bool from_scratch) {
   // a schedule's own grid size is applied on the device (active_blocks)
-  return sched.grid_blocks > 0 ? update_grid_blocks(ctx) : update_blocks_for(ctx, n);
+  return sched.grid_blocks > 0 ? update_grid_blocks(ctx)
+                               : update_blocks_for(ctx, n, m, from_scratch);
 }
 
 void require_intact(const Graph& g) {
@@ -1823,7 +1827,7 @@ void sssp_compute(Context& ctx, Graph& g, Tree& t, dyngb200_stats* st) {
   p.generation = ws.next_generation(1, s);
   p.touch_gen = 1;
   p.heavy_degree = 256;
-  const int blocks = persistent_blocks(ctx, sched, g.n);
+  const int blocks = persistent_blocks(ctx, sched, g.n, g.m, true);
   cudaEvent_t e0, e1;
   DYNGB200_CUDA(cudaEventCreate(&e0));
   DYNGB200_CUDA(cudaEventCreate(&e1));
@@ -1880,7 +1884,8 @@ static double us_since(std::chrono::steady_clock::time_point t0) {
   return std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t0).count();
 }
 
-static void enqueue_attempt(PendingUpdate& u) {
+// `n_after`: the vertices that the batch leaves, as a first attempt found them (0: not known).
+static void enqueue_attempt(PendingUpdate& u, long long n_after = 0) {
   const auto h0 = std::chrono::steady_clock::now();
   Context& ctx = *u.ctx;
   Graph& g = *u.g;
@@ -1891,8 +1896,14 @@ static void enqueue_attempt(PendingUpdate& u) {
   // every allocation of the attempt comes before the applier is queued: a failed one leaves the
   // graph as it was
   g.pinned.reserve(kCounterSlots + g.host_columns.size());
+  // the grid for the graph as the batch leaves it: every insertion may bring an edge and two vertices
+  const long long grown =
+      g.props.allow_vertex_growth ? std::min(g.n + 2 * u.b.ni, g.n_cap) : g.n;
+  u.blocks = persistent_blocks(ctx, u.sched, std::max(grown, n_after),
+                               g.m + u.b.ni * (g.props.directed ? 1 : 2), false);
   DYNGB200_CUDA(cudaEventRecord(u.e0, s));
-  apply_launch(ctx, g, u.b, t.opt.objective, t.opt.delta, &u.sched, &t, u.learned, u.operators);
+  apply_launch(ctx, g, u.b, t.opt.objective, t.opt.delta, &u.sched, &t, u.learned, u.operators,
+               u.blocks);
   DYNGB200_CUDA(cudaEventRecord(u.e1, s));
   u.host_us[1] += us_since(h0);
   const auto h1 = std::chrono::steady_clock::now();
@@ -1939,7 +1950,6 @@ void sssp_update_begin(Context& ctx, Graph& g, Tree& t, const dyngb200_batch& ba
   if (g.host_columns[t.opt.objective].dirty) graph_rescan_columns(ctx, g);
   graph_index_reserve(ctx, g, batch.num_insertions * (g.props.directed ? 1 : 2));
   u.b = stage_batch(ctx, batch, g.k, true);
-  u.blocks = persistent_blocks(ctx, sched, g.n);
   for (cudaEvent_t& e : ctx.update_events)
     if (!e) DYNGB200_CUDA(cudaEventCreate(&e));
   u.e0 = ctx.update_events[0];
@@ -2034,7 +2044,6 @@ void sssp_update_end(PendingUpdate& u, dyngb200_stats* st) {
   Workspace& ws = ctx.ws;
   const Scheduler* learned = u.learned;
   const dyngb200_schedule& sched = u.sched;
-  const int blocks = u.blocks;
   const long long launches0 = u.launches0;
   UpdateCtl r{};
   for (int attempt = 0;; ++attempt) {
@@ -2050,7 +2059,7 @@ void sssp_update_end(PendingUpdate& u, dyngb200_stats* st) {
       // nothing was changed: grow the vertex capacity or the arenas and run again
       graph_grow(ctx, g, r.n_after > g.n_cap ? r.n_after : 0,
                  static_cast<long long>(r.top_out), static_cast<long long>(r.top_in));
-      enqueue_attempt(u);
+      enqueue_attempt(u, r.n_after);
       continue;
     }
     break;
@@ -2089,7 +2098,7 @@ void sssp_update_end(PendingUpdate& u, dyngb200_stats* st) {
   g.n = g.host_counters.n;
   g.m = g.host_counters.m;
   t.version = g.version;
-  finish_tree(ctx, g, t, r, blocks, u.operators, apply_ms, sssp_ms, learned, sched, launches0,
+  finish_tree(ctx, g, t, r, u.blocks, u.operators, apply_ms, sssp_ms, learned, sched, launches0,
               st);
   if (st)
     for (int i = 0; i < 4; ++i) st->host_us[i] = static_cast<float>(u.host_us[i]);
@@ -2163,7 +2172,7 @@ static void sssp_rerun(Context& ctx, Graph& g, Tree& t, const UpdateCtl& applied
   DYNGB200_CUDA(cudaEventCreate(&e1));
   DYNGB200_CUDA(cudaEventCreate(&e2));
   upload_control(ctx, init);
-  const int blocks = persistent_blocks(ctx, sched, g.n);
+  const int blocks = persistent_blocks(ctx, sched, g.n, g.m, false);
   SsspParams p = base_params(ctx, g, t);
   p.from_scratch = 0;
   p.tree_n = t.n;

@@ -260,3 +260,33 @@ def test_pointer_jumping_of_a_graph_at_its_vertex_capacity(blocks):
         back = dict(ins_src=b["del_src"], ins_dst=b["del_dst"], ins_w=np.full(cut.size, 3, np.int32),
                     del_src=empty, del_dst=empty)
         _update(g, og, t, ot, back, "mend", D.sssp.Schedule(grid_blocks=blocks))
+
+
+def test_the_grid_follows_the_edges_and_the_batch():
+    # 600 vertices with 180,000 edges are as much work as a sparse graph of many more vertices; a
+    # batch that brings most of the graph, or names one far vertex, sizes the grid for what it leaves
+    rng = np.random.default_rng(2)
+    n = 600
+    src, dst = rng.integers(0, n, (2, 300 * n)).astype(np.int32)
+    w = rng.integers(1, 1000, src.size).astype(np.int32)
+    g, og, t, ot = _both(n, src, dst, w)
+    full = D.sssp.update(g, D.EdgeBatch(), t, D.sssp.Schedule(grid_blocks=1 << 20)).grid_blocks
+    O.update(og, O.Batch(*_i32([], [], [], [], [])), ot)
+    st = _update(g, og, t, ot, random_batch(rng, n, src, dst, 50, tree_parents=ot.parents), "dense")
+    assert min(full, _edges(g) // 5000) <= st.grid_blocks <= full
+    assert D.sssp.compute(g, 0, stats=True)[1].grid_blocks >= st.grid_blocks
+    chain = np.arange(99, dtype=np.int32)
+    for bring in (40_000, 1):
+        g, og, t, ot = _both(100, chain, chain + 1, np.ones(99, np.int32))
+        top = 200_000
+        src, dst = rng.integers(0, top, (2, bring)).astype(np.int32)
+        src[0], dst[0] = 99, top - 1
+        empty = src[:0]
+        b = dict(ins_src=src, ins_dst=dst, ins_w=rng.integers(1, 9, bring).astype(np.int32),
+                 del_src=empty, del_dst=empty)
+        st = _update(g, og, t, ot, b, "grow")
+        assert st.grid_blocks >= min(full, top // 400)
+
+
+def _edges(g):
+    return int(g.to_csr().row_ptr[-1])

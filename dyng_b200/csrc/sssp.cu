@@ -815,19 +815,24 @@ __device__ __forceinline__ void clear_step(UpdateCtl* c, int it) {
   c->local_rounds[(it + 1) % 3] = 0;
 }
 
-// The invalidation without a schedule's say: a top-down walk of the invalidated subtrees where
-// the changed tree edges are few, pointer jumping otherwise.  Pointer jumping visits every vertex
-// in each of its four to seven rounds (85 us at 4.2M vertices, 20 us at a thousand); the walk
-// reads the out-rows of the invalidated vertices alone, but takes as many levels as their subtrees
-// are deep.  So it is tried on graphs of at least kDenseDegree edges per vertex (shallow trees; on
-// a grid the subtrees are thousands of levels deep) with few roots, and what is not reached after
-// two levels of the grid (six on large graphs, where a round of pointer jumping costs more) is left
-// to pointer jumping.  At R-MAT scale 22 / 1k changes the walk took 8 us in the direction that
-// invalidates 190 vertices and 138 in the one that invalidates 660, pointer jumping 107 in both.
-constexpr long long kWalkRoots = 32;      // or one per kWalkShare vertices where that is more
+// The invalidation without a schedule's say: a small batch's roots are walked down one level, and
+// where that does not reach every invalidated vertex, pointer jumping does.  Most vertices of a
+// dense graph's tree are leaves or nearly, so the few roots of a small batch often have next to
+// nothing below them; pointer jumping costs its passes over every vertex whatever they have (15 us at a
+// thousand vertices, 58 at 1M, 95-112 at 4.2M).  R-MAT scale 22 / 1k changes: 9 us against 95 in the
+// direction whose 191 invalidated vertices are leaves, 117 against 96 in the other; 1,024 vertices
+// / 32 changes: 8 and 5 us against 15.  A walk costs a round trip per vertex of the subtrees' depth
+// and a random parent per slot of their rows, so it stops early: a cut near the source, whose
+// subtree is half the graph, took 476 us with six levels and no bound on their slots, 84 with this,
+// 58 with pointer jumping alone (R-MAT scale 20; scale 22: 594, 141, 110; uniform 3M x 8: 977, 188,
+// 165).  It is tried for at most kWalkRoots roots, or one per kWalkShare vertices; the level may hold
+// kWalkSlots slots per warp of the grid, and a block goes down from it once more by itself where it
+// found at most kTriedLight light rows and kTriedMed medium ones.
+constexpr long long kWalkRoots = 32;
 constexpr long long kWalkShare = 16384;
-constexpr long long kWalkLarge = 1 << 20;  // six levels from here on, two below
 constexpr int kWalkPairs = 2048;  // larger batches hardly hold so few roots: not listed for it
+constexpr int kWalkSlots = 32;
+constexpr int kTriedRounds = 1, kTriedLight = 16, kTriedMed = 1;
 
 // Pointer jumping starts from a sequential pass that lays out every vertex's ancestor, except on
 // graphs of at most kPjShort vertices, whose first round reads the stamps and parents itself: a
@@ -837,18 +842,20 @@ constexpr int kWalkPairs = 2048;  // larger batches hardly hold so few roots: no
 constexpr long long kPjShort = 1LL << 18;
 
 // A block's own levels of the walk: the subtrees below the vertices that it invalidated (a vertex
-// has one tree parent, so no two blocks meet).  What does not fit is shared with the grid.
+// has one tree parent, so no two blocks meet).  What does not fit is shared with the grid.  (These
+// limits: a walk that the schedule names.)
 constexpr int kWalkLight = 256;
 constexpr int kWalkMed = 16;
 constexpr int kWalkRounds = 8;
-__device__ __forceinline__ void local_walk(const SsspParams& p, Ctx& X) {
+__device__ __forceinline__ void local_walk(const SsspParams& p, Ctx& X, int max_rounds,
+                                           int max_light, int max_med) {
   __shared__ int s_own[kWalkLight + kWalkMed];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int kWarps = kThreads / 32;
   for (int round = 0;; ++round) {
     __syncthreads();
     const int nl = g_stage.cnt[kStNext], nm = g_stage.cnt[kStNextMed];
-    if (nl + nm == 0 || nl > kWalkLight || nm > kWalkMed || round >= kWalkRounds) return;
+    if (nl + nm == 0 || nl > max_light || nm > max_med || round >= max_rounds) return;
     if (static_cast<int>(threadIdx.x) < nl) s_own[threadIdx.x] = g_stage.data[kStNext][threadIdx.x];
     if (static_cast<int>(threadIdx.x) < nm)
       s_own[kWalkLight + threadIdx.x] = g_stage.data[kStNextMed][threadIdx.x];
@@ -1162,10 +1169,15 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
         const int mc = ld_cg(&c->walk_med_cnt[cs]);
         const u64 hc = ld_cg(&c->walk_heavy[cs]);
         if (nc == 0 && mc == 0 && (hc >> 40) == 0) break;
-        if (!p.walk && level >= (n >= kWalkLarge ? 6 : 2)) {
-          // too deep: pointer jumping finishes it
-          walked = false;
-          break;
+        if (!p.walk) {
+          // rows at their class's longest, heavy ones by their chunks
+          const long long slots =
+              static_cast<long long>(kLightMax) * nc + static_cast<long long>(p.heavy_degree) * mc +
+              kHeavyChunk * static_cast<long long>(hc & ((1ULL << 40) - 1));
+          if (level > 0 || slots > kWalkSlots * nwarps) {
+            walked = false;  // too deep or too wide: pointer jumping finishes it
+            break;
+          }
         }
         if (level > n + 1) {
           if (tid == 0) atomicOr(&c->error, kErrNotConverged);
@@ -1184,7 +1196,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
         const int cb = level & 1;
         expand<kWalk>(p, X, cb ? p.near_b : p.near_a, nc, cb ? p.near_med_b : p.near_med_a, mc,
                       cb ? p.heavy_b : p.heavy_a, hc, gwarp, nwarps);
-        local_walk(p, X);
+        local_walk(p, X, p.walk ? kWalkRounds : kTriedRounds, p.walk ? kWalkLight : kTriedLight,
+                   p.walk ? kWalkMed : kTriedMed);
         if (!grid_barrier(c, bar)) return;
         ++level;
       }

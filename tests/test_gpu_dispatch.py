@@ -6,7 +6,8 @@ against the oracle bit for bit:
   - threshold raises that find nothing below the new threshold and skip to the next distance;
   - relocated rows around the length above which a row moves in chunks;
   - host batches around the size that comes over with the control block;
-  - the subtree walk that an update without a schedule tries when few tree edges changed;
+  - the subtree walk that an update without a schedule tries when few tree edges changed: its
+    limits in roots, batch, depth and width;
   - pointer jumping on either side of the size up to which it starts without a seeding pass, and
     on a graph that fills its vertex capacity.
 """
@@ -208,9 +209,51 @@ def test_few_changed_tree_edges(roots, depth):
              del_src=heads[pick].astype(np.int32), del_dst=first[pick].astype(np.int32))
     st = _update(g, og, t, ot, b, "cut")
     assert st.invalidated == roots * depth
+    assert st.invalidation == (1 if roots <= 32 and depth == 1 else 0)
     back = dict(ins_src=b["del_src"], ins_dst=b["del_dst"], ins_w=np.full(roots, 3, np.int32),
                 del_src=empty, del_dst=empty)
     _update(g, og, t, ot, back, "mend")
+
+
+@pytest.mark.parametrize("n", [9000, 60_000])
+def test_a_cut_edge_above_most_of_the_tree_is_not_walked(n):
+    # the source reaches a hub, and the hub nearly every vertex: its row is wider than a level of
+    # the walk may be (32 slots per warp of 24 and 157 blocks), so nothing of it is walked
+    rng = np.random.default_rng(n)
+    v = np.arange(2, n)
+    far = rng.integers(2, n, (2, 8 * n))
+    src = np.concatenate([[0, 0], np.ones(n - 2), far[0]])
+    dst = np.concatenate([[1, 2], v, far[1]])
+    w = np.concatenate([[1, 10**6], rng.integers(1, 9, n - 2), rng.integers(10, 1000, 8 * n)])
+    src, dst, w = _i32(src, dst, w)
+    g, og, t, ot = _both(n, src, dst, w)
+    cut = dict(zip(("ins_src", "ins_dst", "ins_w", "del_src", "del_dst"), _i32([], [], [], [0], [1])))
+    st = _update(g, og, t, ot, cut, "cut")
+    rows = st.work[D.sssp.Stats.WORK_NAMES.index("walk_rows")]
+    assert st.invalidated >= n - 2
+    assert st.invalidation == 0 and rows == 0
+
+
+@pytest.mark.parametrize("roots,pairs", [(64, 2048), (65, 2048), (64, 2049), (20, 900)])
+def test_the_walks_limits_on_a_large_graph(roots, pairs):
+    # 2^20 vertices, one root per 16,384 allowed: leaves cut off, with other changes around them
+    rng = np.random.default_rng(roots)
+    n, leaves = 1 << 20, 100
+    core = n - leaves
+    src = np.concatenate([rng.integers(0, core, 7 * n), rng.integers(0, core, leaves)])
+    dst = np.concatenate([rng.integers(0, core, 7 * n), np.arange(core, n)])
+    w = rng.integers(1, 1000, src.size)
+    src, dst, w = _i32(src, dst, w)
+    g, og, t, ot = _both(n, src, dst, w)
+    assert (ot.parents[core:] >= 0).sum() >= roots
+    cut = core + np.nonzero(ot.parents[core:] >= 0)[0][:roots]
+    other = rng.choice(core, pairs - roots, replace=False)  # heavy loops: no tree edge changes
+    loop = np.full(other.size, 10**6)
+    b = dict(zip(("ins_src", "ins_dst", "ins_w", "del_src", "del_dst"),
+                 _i32(other, other, loop, ot.parents[cut], cut)))
+    st = _update(g, og, t, ot, b, "cut")
+    assert st.invalidated == roots
+    assert st.invalidation == (1 if roots <= 64 and pairs <= 2048 else 0)
 
 
 @pytest.mark.parametrize("depth", [1, 2, 3, 4, 40, 3000])

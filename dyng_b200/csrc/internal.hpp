@@ -370,7 +370,7 @@ struct Graph {
 struct TreeHistory {
   long long invalidated;
   int frontier[4];  // sizes of the first four near-far steps
-  int iterations;   // near-far iterations + epochs
+  int steps;        // near-far steps, threshold raises among them
   int rounds;       // pointer-jumping rounds
 };
 

@@ -106,7 +106,7 @@ static __device__ __forceinline__ void infer_schedule_block(const InferArgs& a, 
     f[8] = lg(static_cast<double>(h.invalidated));
     f[9] = lg(static_cast<double>(abs(h.frontier[0])));
     f[10] = lg(static_cast<double>(abs(fmax)));
-    f[11] = lg(static_cast<double>(h.iterations));
+    f[11] = lg(static_cast<double>(h.steps));
   }
   __syncthreads();
   if (lane < kMlpIn) c->features[lane] = f[lane];

@@ -493,7 +493,7 @@ __global__ void k_op_finish(SsspParams p, OpSummary s) {
     TreeHistory h{};
     h.invalidated = c->invalidated;
     for (int i = 0; i < 4; ++i) h.frontier[i] = s.frontier[i];
-    h.iterations = s.iterations + s.epochs;
+    h.steps = s.iterations + s.epochs;
     h.rounds = s.rounds;
     *p.hist = h;
   }

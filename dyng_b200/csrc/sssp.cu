@@ -693,7 +693,8 @@ __device__ __forceinline__ void invalidate(const SsspParams& p, int v) {
 // State of the near-far loop (the same in every block).
 struct LoopState {
   int gen;
-  int it;           // steps of the grid so far (selects the list buffers and counter slots)
+  int it;           // steps of the grid so far, raises among them (selects the list buffers and
+                    // counter slots)
   int iterations;   // push rounds: the steps, and the rounds the blocks ran inside them
   int epochs;       // threshold raises (select the far pile's buffers and counter slots)
   bool split_empty; // the last threshold raise brought no vertex below the threshold
@@ -912,12 +913,11 @@ __device__ bool near_far(const SsspParams& p, Ctx& X, LoopState& S, unsigned& ba
     const bool near_work = nc > 0 || mc > 0 || (hc >> 40) > 0;
     if (!near_work && far_count == 0) return true;
     int* far = (S.epochs & 1) ? p.far_b : p.far_a;
-    const int step = S.iterations + S.epochs;
-    if (leader && step < 64) {
-      c->trace_n[step] = near_work ? nc + mc : -far_count;
-      c->trace_h[step] = static_cast<int>(hc & 0xffffffffu);
-      c->trace_t[step] = static_cast<unsigned>(global_ns() - c->phase_ns[0]);
-      c->trace_len = step + 1;
+    if (leader && S.it < 64) {
+      c->trace_n[S.it] = near_work ? nc + mc : -far_count;
+      c->trace_h[S.it] = static_cast<int>(hc & 0xffffffffu);
+      c->trace_t[S.it] = static_cast<unsigned>(global_ns() - c->phase_ns[0]);
+      c->trace_len = S.it + 1;
     }
     if (S.gen > kMaxGeneration - kLocalRounds - 8) {
       // the claims would run out of generations: start them over
@@ -953,11 +953,11 @@ __device__ bool near_far(const SsspParams& p, Ctx& X, LoopState& S, unsigned& ba
       // share a flush
       const long long gwarp =
           local ? static_cast<long long>(threadIdx.x >> 5) * g_nblk + blockIdx.x : tid >> 5;
-      const unsigned long long t_busy = step == 0 ? global_ns() : 0;
+      const unsigned long long t_busy = S.it == 0 ? global_ns() : 0;
       expand<kPush>(p, X, lists[S.it & 1], nc, mlists[S.it & 1], mc, hlists[S.it & 1], hc, gwarp,
-                    nwarps, step == 0 ? &c->work[16] : nullptr, &c->med_cursor[cs],
+                    nwarps, S.it == 0 ? &c->work[16] : nullptr, &c->med_cursor[cs],
                     &c->heavy_cursor[cs]);
-      if (step == 0) {
+      if (S.it == 0) {
         // balance of the first step: the slowest warp's and the summed busy time, and warps
         // (met per block in shared memory: one global atomic per block and value)
         __shared__ long long s_busy[2];
@@ -1512,7 +1512,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
   LoopState S{gen, 0, 0, 0, false, X.threshold};
   if (!near_far(p, X, S, bar, delta, n, p.small_frontier)) return;
   gen = S.gen;
-  const int iterations = S.iterations, epochs = S.epochs;
+  const int iterations = S.iterations, epochs = S.epochs, steps = S.it;
   if (tid == 0) c->phase_ns[6] = global_ns();
 
   // ---- commit: unpack (fused.cuh:419-494) ------------------------------------------------------
@@ -1641,7 +1641,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
       h.invalidated = ld_cg(&c->invalidated);
       const int len = ld_cg(&c->trace_len);
       for (int i = 0; i < 4; ++i) h.frontier[i] = i < len ? ld_cg(&c->trace_n[i]) : 0;
-      h.iterations = iterations + epochs;
+      h.steps = steps;
       h.rounds = ld_cg(&c->rounds);
       *p.hist = h;
     }

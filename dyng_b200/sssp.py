@@ -135,7 +135,8 @@ class Stats:
 
     @property
     def trace(self) -> tuple:
-        """(light, heavy chunks, start us) per near-far step; light < 0: an epoch."""
+        """(light and medium rows, heavy chunks, start us) per step of the near-far loop (the first
+        64); a negative first entry: a threshold raise over that many far vertices."""
         s = self._s
         return tuple((int(s.trace_light[i]), int(s.trace_heavy[i]), float(s.trace_us[i]))
                      for i in range(min(int(s.trace_len), 64)))

@@ -106,8 +106,9 @@ typedef struct dyngb200_stats {
   dyngb200_apply_summary batch;
   int64_t invalidated; /* deterministic */
   int64_t affected;    /* deterministic: vertices whose distance or parent changed */
-  int64_t iterations;  /* schedule-dependent */
-  int64_t epochs;      /* schedule-dependent */
+  int64_t iterations;  /* push rounds: steps of the grid, and the most rounds that a block ran by
+                        * itself inside each; schedule- and timing-dependent */
+  int64_t epochs;      /* threshold raises; schedule-dependent */
   int64_t pushes;      /* schedule-dependent */
   int32_t packed_parents;
   int32_t engine_used; /* dyngb200_engine that ran: FUSED or OPERATORS */
@@ -134,11 +135,10 @@ typedef struct dyngb200_stats {
   /* Device time of the kernel's phases (ms): setup+roots, pointer jumping, invalidation, pull,
    * first split, near-far loop, unpack. */
   float phase_ms[7];
-  /* Trace of the first 64 steps of the near-far loop: light frontier size (negative: an epoch
-   * with that many far vertices), heavy chunks, and the step's start in microseconds since the
-   * kernel began. */
-  /* The first 64 near-far steps: light frontier entries, heavy-row chunks (bit 30 set: the step
-   * ran block-local, in the small-frontier mode), and the time since the kernel began. */
+  /* The first 64 steps of the near-far loop (the rounds that blocks run inside a step have none
+   * of their own): frontier entries of light and medium rows (negative: a threshold raise over that
+   * many far vertices), chunks of heavy rows, and the step's start in microseconds since the kernel
+   * began. */
   int32_t trace_len;
   int32_t trace_light[64];
   int32_t trace_heavy[64];

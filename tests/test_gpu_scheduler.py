@@ -135,6 +135,38 @@ def test_device_features_of_a_hand_case(D):
     assert st2.features[11] == pytest.approx(np.log2(1 + st.iterations + st.epochs))
 
 
+def test_trace_and_history_of_an_update_with_rounds_inside_its_steps(D):
+    # a grid's repair runs dozens of the blocks' own rounds; the trace has a row per step of the
+    # whole grid, none of them empty, and the history that the next update's features show is its
+    side = 200
+    v = np.arange(side * side)
+    right, down = v[v % side + 1 < side], v[v < side * (side - 1)]
+    s = np.concatenate([right, right + 1, down, down + side]).astype(np.int32)
+    d = np.concatenate([right + 1, right, down + side, down]).astype(np.int32)
+    w = np.random.default_rng(4).integers(1, 50, s.size).astype(np.int32)
+    g = D.Graph.from_edges(s, d, w, num_vertices=side * side)
+    tree = D.sssp.compute(g, 0)
+    seen = False
+    for cut in (side, 0, 77 * side + 78, 120 * side + 9):
+        st = D.sssp.update(g, D.EdgeBatch.from_arrays([], [], [], s[s == cut], d[s == cut]), tree)
+        trace = st.trace
+        steps = len(trace)
+        assert all(light != 0 or heavy != 0 for light, heavy, _ in trace)
+        assert all(a[2] <= b[2] for a, b in zip(trace, trace[1:]))
+        seen |= st.iterations + st.epochs > steps and 2 < steps < 64
+        again = D.sssp.update(g, D.EdgeBatch.from_arrays(s[s == cut], d[s == cut], w[s == cut]), tree,
+                              schedule=D.sssp.Schedule(record_features=True))
+        assert again.features[8] == pytest.approx(np.log2(1 + st.invalidated))
+        sizes = [abs(light) for light, _, _ in trace[:4]] + [0] * 4
+        assert again.features[9] == pytest.approx(np.log2(1 + sizes[0]))
+        # the largest of three signed entries: a raise counts as minus its far vertices
+        signed = ([light for light, _, _ in trace[:4]] + [0] * 4)[1:4]
+        assert again.features[10] == pytest.approx(np.log2(1 + abs(max([0] + signed))))
+        if steps < 64:
+            assert again.features[11] == pytest.approx(np.log2(1 + steps))
+    assert seen
+
+
 def test_learned_updates_equal_plain_updates(D):
     from dyng_b200 import scheduler as S
     rng = np.random.default_rng(9)

@@ -203,7 +203,7 @@ struct Ctx {
   Packing pk;
   u64 maxd;
   u64 threshold;
-  u64 low;       // pull: the smallest distance an offer of this thread brought into the frontier
+  u64 low;       // pull: the smallest distance of the owners that this thread's offers reached
   int gen;       // claim generation of the appends
   ListSet next;  // push: next near frontier; walk: next level; pull: the frontier (light only)
   int* far;
@@ -272,8 +272,10 @@ __device__ __forceinline__ void offer_owner(const SsspParams& p, Ctx& X, int own
   if (cand < old) {
     ++X.atomics;
     touch(p, owner);
-    X.low = min(X.low, X.pk.dist(cand));
   }
+  // in a frontier that another offer of the same owner made, too; an owner that was not invalidated
+  // (heads of a tree that is not canonical) joins with the word that it had
+  if (cand < old || claimed) X.low = min(X.low, X.pk.dist(min(cand, old)));
   if (claimed) {
     ++X.appends;
     staged_append(kStNext, X.next.light, X.next.light_cnt, owner);
@@ -1482,7 +1484,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
       pull_atomics = Y.atomics;
       pull_appends = Y.appends;
       X.tries += Y.tries;
-      // the frontier's smallest distance: every word in it was brought by one of these offers
+      // the frontier's smallest distance: one of these offers brought each of its vertices
       block_min_into(Y.low, &c->minimum);
     }
     if (!grid_barrier(c, bar)) return;

@@ -333,3 +333,25 @@ def test_the_grid_follows_the_edges_and_the_batch():
 
 def _edges(g):
     return int(g.to_csr().row_ptr[-1])
+
+
+@pytest.mark.parametrize("delta", [1, 700, 0])
+def test_heads_that_do_not_improve_start_the_threshold_at_their_distance(delta):
+    # a tree kept as it was imported (not canonical): its insertion heads are pulled and pushed even
+    # if the inserted edge brings them nothing; the first threshold lies above the smallest of them
+    n = 400
+    v = np.arange(1, n, dtype=np.int32)
+    w = np.full(n - 1, 1000, np.int32)
+    g, og, _, _ = _both(n, v - 1, v, w)
+    t = D.sssp.Result.from_arrays(g, 0, np.arange(n) * 1000, np.arange(-1, n - 1), canonicalize=False)
+    heads = np.asarray([310, 200, 350], np.int32)
+    far = np.full(3, 2**30, np.int32)
+    b = D.EdgeBatch.from_arrays(np.zeros(3, np.int32), heads, far, [], [])
+    st = D.sssp.update(g, b, t, D.sssp.Schedule(delta=delta))
+    np.testing.assert_array_equal(t.distances, np.arange(n) * 1000)
+    np.testing.assert_array_equal(t.parents, np.arange(-1, n - 1))
+    assert st.affected == 0
+    width = st.delta
+    raises = 0 if width > 150_000 else 4  # the other heads lie 110 and 150 edges on
+    assert st.epochs <= raises
+    assert st.trace[0][0] > 0  # the nearest head is pushed by the first step, without a raise

@@ -1893,6 +1893,12 @@ int Workspace::next_generation(int count, cudaStream_t s) {
   return g;
 }
 
+void Workspace::forget_marks(cudaStream_t s) {
+  for (DevBuf<int>* b : {&stamp, &near_stamp, &touch_stamp, &in_far})
+    DYNGB200_CUDA(cudaMemsetAsync(b->ptr, 0, b->count * sizeof(int), s));
+  generation = 0;
+}
+
 int Workspace::next_touch_generation(cudaStream_t s) {
   if (touch_generation > INT32_MAX / 2) {
     DYNGB200_CUDA(cudaMemsetAsync(touch_out_stamp.ptr, 0, touch_out_stamp.count * sizeof(int), s));

@@ -264,6 +264,8 @@ struct Workspace {
   void reserve_vertices(long long n_cap, cudaStream_t s);
   void reserve_batch(long long ops, int k, cudaStream_t s);
   int next_generation(int count, cudaStream_t s);  // reserves `count` sssp generations
+  // After a kernel that stopped part-way: its stamps and far marks belong to no later call.
+  void forget_marks(cudaStream_t s);
   int next_touch_generation(cudaStream_t s);
 };
 

@@ -1859,6 +1859,7 @@ void sssp_compute(Context& ctx, Graph& g, Tree& t, dyngb200_stats* st) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   const UpdateCtl& r = *ws.host_ctl.ptr;
+  if (r.error & (kErrTimeout | kErrNotConverged)) ws.forget_marks(s);
   if (r.error & kErrTimeout) throw Error(DYNGB200_INTERNAL, "sssp: a grid barrier timed out");
   if (r.error & kErrNotConverged)
     throw Error(DYNGB200_INTERNAL, "sssp: the near-far loop did not converge");
@@ -2001,6 +2002,7 @@ static void finish_tree(Context& ctx, Graph& g, Tree& t, const UpdateCtl& r, int
                 "reach a root in ceil(log2 n) + 1 rounds)");
   }
   if (r.error & (kErrTimeout | kErrNotConverged)) {
+    ctx.ws.forget_marks(ctx.stream);
     t.poisoned = true;
     throw Error(DYNGB200_INTERNAL, (r.error & kErrTimeout)
                                        ? "sssp::update: a grid barrier timed out"

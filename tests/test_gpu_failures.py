@@ -3,7 +3,8 @@
   - a grid barrier that never completes (a phantom block that never arrives, with a short
     test-only time limit): every block leaves the kernel and the call reports INTERNAL; in the
     batch applier before any change (graph and tree unchanged), in the sssp kernel after the
-    batch was applied (the tree poisoned); the context keeps working either way;
+    batch was applied (the tree poisoned), or part-way through its loop; the context keeps working
+    either way, and no mark of the stopped call is taken for one of the next;
   - a long loop run by one block while the others wait at a grid barrier outlives that limit
     without a timeout: the waiting blocks restart their limit whenever the working block shows
     progress;
@@ -93,6 +94,32 @@ def test_a_barrier_of_the_sssp_kernel_that_never_completes_times_out_and_poisons
     fresh = D.sssp.compute(g, 0)
     np.testing.assert_array_equal(fresh.distances, ot.distances)
     np.testing.assert_array_equal(fresh.parents, ot.parents)
+
+
+def test_a_call_that_timed_out_late_leaves_no_marks_for_the_next():
+    # with distances too long to pack a parent beside, the commit walks a hub's row of a million
+    # slots in one thread while the other blocks wait: with a limit of 50 us they give up there,
+    # after the near-far loop has stamped every vertex.  Those stamps name the same step as a solve
+    # from the hub itself would (from vertex 0 the hub's neighbours come one step later)
+    n = (1 << 20) + 2
+    v = np.arange(2, n)
+    src = np.concatenate([[0], np.ones(n - 2), [n - 1]]).astype(np.int32)
+    dst = np.concatenate([[1], v, [0]]).astype(np.int32)
+    w = np.concatenate([[1], np.ones(n - 2), [2**31 - 1]]).astype(np.int32)
+    res = D.Resources(0)
+    g = D.Graph.from_edges(src, dst, w, n, resources=res)
+    res.set_test_hooks(barrier_timeout_ns=50_000)
+    try:
+        with pytest.raises(D.InternalError, match="timed out"):
+            D.sssp.compute(g, 0)
+    finally:
+        res.set_test_hooks()
+    t, st = D.sssp.compute(g, 1, stats=True)
+    assert not st.packed_parents
+    want = np.ones(n, np.int64)
+    want[1] = 0
+    want[0] = 2**31
+    np.testing.assert_array_equal(t.distances, want)
 
 
 def test_progress_keeps_a_long_single_block_loop_alive():

@@ -479,7 +479,7 @@ __device__ __forceinline__ int matches_before(unsigned m, int* all) {
   return incl - __popc(m);
 }
 
-// Multi-edge graphs: one thread per pair walks its rows in order (the first alive matches).
+// Multi-edge graphs: a warp per pair walks its rows in order (the first alive matches).
 // Records c, the first match and the match the insertions address (see resolve).
 __device__ void ph_scan_multi(const ApplyParams& p, long long tid, long long threads) {
   // one warp per pair: the lanes read a row kScanSlots at a time and rank the matches
@@ -1818,7 +1818,7 @@ void Workspace::reserve_vertices(long long n_cap, cudaStream_t s) {
     DYNGB200_CUDA(cudaMemsetAsync(b->ptr, 0, n * sizeof(int), s));
   }
   for (DevBuf<int>* b : {&row_slot_out, &row_slot_in, &ancestor, &candidates, &frontier, &near_a,
-                         &near_b, &far_a, &far_b, &touched, &cand_med, &near_med_a, &near_med_b}) {
+                         &near_b, &far_a, &far_b, &cand_med, &near_med_a, &near_med_b}) {
     b->release();
     b->reserve(n, s);
   }

@@ -154,7 +154,6 @@ struct UpdateCtl {
   int med_cursor[3];
   int local_rounds[3];  // the most rounds a block ran by itself inside a push step (same slots)
   unsigned long long heavy_cursor[3];
-  int touched_count;
   int active[3];
   int rounds;
   int iterations, epochs;
@@ -250,7 +249,7 @@ struct Workspace {
   DevBuf<int> pj_blk;  // per-block survivor counts of pointer jumping
   DevBuf<long long> batch_extrema;  // update_each: per-objective insertion weight range, max id
   DevBuf<int> candidates, frontier, near_a, near_b, far_a, far_b, heavy_a, heavy_b, pull_heavy,
-      touched, cand_med, near_med_a, near_med_b;
+      cand_med, near_med_a, near_med_b;
   DevBuf<UpdateCtl> ctl;
   HostBuf<UpdateCtl> host_ctl;
   DevBuf<unsigned long long> op_counts;  // the operators engine's step counters

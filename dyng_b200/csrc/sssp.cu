@@ -43,10 +43,10 @@ __device__ __forceinline__ unsigned ld_volatile(const unsigned* p) { return gs_l
 // the stage to the global list with ONE global atomicAdd for its slot range, so the global list
 // counters see one atomic per block and phase instead of one per warp group.  A full stage falls
 // back to the global list directly.  Stages: the next frontier (near list, pull frontier or walk
-// level), the far pile, the touched list and the pull candidates.
-constexpr int kStages = 6;
+// level), the far pile and the pull candidates.
+constexpr int kStages = 5;
 constexpr int kStageCap = 768;
-enum StageId { kStNext = 0, kStFar = 1, kStTouched = 2, kStCand = 3, kStNextMed = 4, kStCandMed = 5 };
+enum StageId { kStNext = 0, kStFar = 1, kStCand = 2, kStNextMed = 3, kStCandMed = 4 };
 
 struct StageSet {
   int cnt[kStages];
@@ -1790,7 +1790,6 @@ static SsspParams base_params(Context& ctx, Graph& g, Tree& t) {
   p.cand_med = ws.cand_med.ptr;
   p.near_med_a = ws.near_med_a.ptr;
   p.near_med_b = ws.near_med_b.ptr;
-  p.touched = ws.touched.ptr;
   p.ctl = ws.ctl.ptr;
   p.hist = t.hist.ptr;
   expects(ws.pj_blk.ptr != nullptr, "sssp: the workspace was not reserved", DYNGB200_INTERNAL);
@@ -2363,9 +2362,9 @@ void tree_repack(Context& ctx, Tree& t, int bits) {
 // kStaticScratchBytes that every GPU which loads this library holds until the process exits.
 // ------------------------------------------------------------------------------------------------
 constexpr long long kStaticMaxVertices = 1LL << 16;
-// control block + packed words (8 B) + 15 int lists / stamp arrays + 3 int2 lists, per vertex
+// control block + packed words (8 B) + 14 int lists / stamp arrays + 3 int2 lists, per vertex
 constexpr long long kStaticScratchBytes =
-    4096 + kStaticMaxVertices * (8 + 15 * 4 + 3 * 8);
+    4096 + kStaticMaxVertices * (8 + 14 * 4 + 3 * 8);
 
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
 
@@ -2417,7 +2416,7 @@ void sssp_compute_static(Graph& g, int32_t source, int objective, long long delt
   auto* ctl = reinterpret_cast<UpdateCtl*>(base);
   auto* packed = reinterpret_cast<u64*>(base + 4096);
   int* ints = reinterpret_cast<int*>(base + 4096 + 8 * N);
-  int2* pairs = reinterpret_cast<int2*>(base + 4096 + 8 * N + 15 * 4 * N);
+  int2* pairs = reinterpret_cast<int2*>(base + 4096 + 8 * N + 14 * 4 * N);
   SsspParams p{};
   p.g = g.view();
   p.objective = objective;
@@ -2437,10 +2436,9 @@ void sssp_compute_static(Graph& g, int32_t source, int objective, long long delt
   p.near_b = ints + 8 * N;
   p.far_a = ints + 9 * N;
   p.far_b = ints + 10 * N;
-  p.touched = ints + 11 * N;
-  p.cand_med = ints + 12 * N;
-  p.near_med_a = ints + 13 * N;
-  p.near_med_b = ints + 14 * N;
+  p.cand_med = ints + 11 * N;
+  p.near_med_a = ints + 12 * N;
+  p.near_med_b = ints + 13 * N;
   p.heavy_a = pairs;
   p.heavy_b = pairs + N;
   p.pull_heavy = pairs + 2 * N;

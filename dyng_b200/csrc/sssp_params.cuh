@@ -45,7 +45,6 @@ struct SsspParams {
   int* cand_med;
   int* near_med_a;
   int* near_med_b;
-  int* touched;
   int generation;
   int touch_gen;
   int heavy_degree;

@@ -4,7 +4,8 @@ against the oracle bit for bit:
   - near-far steps that a block continues by itself: short frontiers of light rows, the hand-over
     back to the grid, a chain longer than the claims' generations last;
   - threshold raises that find nothing below the new threshold and skip to the next distance;
-  - relocated rows around the length above which a row moves in chunks;
+  - relocated rows around the length above which a row moves in chunks, and rows around the length
+    above which the index build and the compaction cut them;
   - host batches around the size that comes over with the control block;
   - the subtree walk that an update without a schedule tries when few tree edges changed: its
     limits in roots, batch, depth and width;
@@ -21,6 +22,7 @@ from tests.helpers import random_batch
 pytestmark = pytest.mark.gpu
 
 MOVE_CHUNK = 512          # slots of a row that move as one piece
+LONG_ROW = 1024           # slots of a row that the storage passes take as one piece
 PJ_SHORT = 1 << 18        # vertices up to which pointer jumping starts from the tree itself
 STAGED_VALUES = 64 * 1024 // 4  # values of a host batch that come over with the control block
 
@@ -162,6 +164,52 @@ def test_relocated_rows_around_the_chunk_length(kind, length):
     # the moved edges are found again (the edge index followed them)
     again = dict(ins_src=src[:0], ins_dst=dst[:0], ins_w=w[:0], del_src=src[~gone], del_dst=dst[~gone])
     _update(g, og, t, ot, again, "delete the moved edges")
+    _csr_same(g, og)
+
+
+@pytest.mark.parametrize("kind", ["sorted", "append", "multi"])
+def test_index_build_and_compaction_of_long_rows(kind):
+    # hubs with rows around one, two and five pieces on either side, churned until the abandoned
+    # slots pass half the edges and the next overflow compacts: a third of every hub's edges go and
+    # as many come, so its row holds tombstones in every piece when the pass reads it
+    rng = np.random.default_rng(17)
+    n = 5 * LONG_ROW + 200
+    lengths = [1, 31, LONG_ROW - 1, LONG_ROW, LONG_ROW + 1, LONG_ROW + 32, 2 * LONG_ROW - 1,
+               2 * LONG_ROW, 2 * LONG_ROW + 1, 5 * LONG_ROW]
+    hubs = 2 + np.arange(len(lengths))
+    far = [100 + rng.permutation(n - 100)[:size] for size in lengths]
+    src = np.concatenate([[0] * hubs.size, *[np.full(f.size, h) for h, f in zip(hubs, far)],
+                          *[f for f in far]])
+    dst = np.concatenate([hubs, *far, *[np.full(f.size, 50 + h) for h, f in zip(hubs, far)]])
+    src, dst, w = _i32(src, dst, rng.integers(1, 100, src.size))
+    props = dict(sorted=kind == "sorted", allow_multi=kind == "multi")
+    g, og, t, ot = _both(n, src, dst, w, D.GraphProperties(**props), O.default_props(
+        sorted=int(props["sorted"]), allow_multi=int(props["allow_multi"])))
+    builds = g.storage()["index_builds"]
+    for step in range(60):
+        gone = [f[rng.random(f.size) < 1 / 3] for f in far]
+        come = [100 + rng.permutation(n - 100)[:x.size + 8] for x in gone]
+        far = [np.unique(np.concatenate([np.setdiff1d(f, x), c])) for f, x, c in zip(far, gone, come)]
+        pairs = lambda lists: (  # noqa: E731
+            np.concatenate([*[np.full(x.size, h) for h, x in zip(hubs, lists)], *lists]),
+            np.concatenate([*lists, *[np.full(x.size, 50 + h) for h, x in zip(hubs, lists)]]))
+        i, j = pairs(come)
+        b = dict(zip(("ins_src", "ins_dst", "ins_w", "del_src", "del_dst"),
+                     _i32(i, j, rng.integers(1, 100, i.size), *pairs(gone))))
+        _update(g, og, t, ot, b, f"step {step}")
+        if g.storage()["compactions"] >= 2:
+            break
+    st = g.storage()
+    assert st["compactions"] >= 2, st
+    assert kind == "multi" or st["index_builds"] > builds
+    _csr_same(g, og)
+    # every edge is found through the rebuilt index
+    csr = og.to_csr()
+    rows = np.repeat(np.arange(n), np.diff(csr["row_ptr"]))
+    some = rng.permutation(rows.size)[:4000]
+    b = dict(zip(("ins_src", "ins_dst", "ins_w", "del_src", "del_dst"),
+                 _i32([], [], [], rows[some], np.asarray(csr["col"])[some])))
+    _update(g, og, t, ot, b, "delete")
     _csr_same(g, og)
 
 

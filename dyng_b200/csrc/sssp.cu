@@ -818,24 +818,27 @@ __device__ __forceinline__ void clear_step(UpdateCtl* c, int it) {
   c->local_rounds[(it + 1) % 3] = 0;
 }
 
-// The invalidation without a schedule's say: a small batch's roots are walked down one level, and
-// where that does not reach every invalidated vertex, pointer jumping does.  Most vertices of a
-// dense graph's tree are leaves or nearly, so the few roots of a small batch often have next to
-// nothing below them; pointer jumping costs its passes over every vertex whatever they have (15 us at a
-// thousand vertices, 58 at 1M, 95-112 at 4.2M).  R-MAT scale 22 / 1k changes: 9 us against 95 in the
-// direction whose 191 invalidated vertices are leaves, 117 against 96 in the other; 1,024 vertices
-// / 32 changes: 8 and 5 us against 15.  A walk costs a round trip per vertex of the subtrees' depth
-// and a random parent per slot of their rows, so it stops early: a cut near the source, whose
-// subtree is half the graph, took 476 us with six levels and no bound on their slots, 84 with this,
-// 58 with pointer jumping alone (R-MAT scale 20; scale 22: 594, 141, 110; uniform 3M x 8: 977, 188,
-// 165).  It is tried for at most kWalkRoots roots, or one per kWalkShare vertices; the level may hold
-// kWalkSlots slots per warp of the grid, and a block goes down from it once more by itself where it
-// found at most kTriedLight light rows and kTriedMed medium ones.
+// The invalidation without a schedule's say: the subtrees of a small batch's roots are walked from
+// one level of the grid, and where that does not reach every invalidated vertex, pointer jumping
+// does.  Most of a dense graph's tree has next to nothing below it, while pointer jumping costs its
+// passes over every vertex whatever the roots have: 15 us at a thousand vertices, 26 at 131,072, 45
+// at 1M, 95 at 4.2M, against 5-15, 8-26, 8-37 and 8-37 us for the walks of batches of 30 to 1,000
+// changes there.  A walk pays a round trip for every level of the subtrees and a random parent per
+// slot of their rows, so it has to stop early.  The level of the grid may hold kWalkSlots slots per
+// warp; a block goes on from it while it holds at most kTriedLight light rows and kTriedMed medium
+// ones, for tried_rounds rounds: what a walk that is given up costs (13-35 us) then stays below what
+// the later rounds of pointer jumping gained, and a cut near the source, whose subtree is half the
+// graph, takes 82 us at R-MAT scale 20 (58 with pointer jumping alone, 476 with six levels without a
+// bound), 172 at scale 22 (110, 594) and 198 on a uniform graph of 3M x 8 edges (165, 977).  At most
+// kWalkRoots roots are walked from, or one per kWalkShare vertices where that is more.
 constexpr long long kWalkRoots = 32;
 constexpr long long kWalkShare = 16384;
 constexpr int kWalkPairs = 2048;  // larger batches hardly hold so few roots: not listed for it
 constexpr int kWalkSlots = 32;
-constexpr int kTriedRounds = 1, kTriedLight = 16, kTriedMed = 1;
+constexpr int kTriedLight = 128, kTriedMed = 8;
+__device__ __forceinline__ int tried_rounds(long long n) {
+  return n >= (1 << 20) ? 8 : (n >= (1 << 17) ? 6 : 4);
+}
 
 // Pointer jumping starts from a sequential pass that lays out every vertex's ancestor, except on
 // graphs of at most kPjShort vertices, whose first round reads the stamps and parents itself: a
@@ -1198,7 +1201,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_sssp(SsspParams p) {
         const int cb = level & 1;
         expand<kWalk>(p, X, cb ? p.near_b : p.near_a, nc, cb ? p.near_med_b : p.near_med_a, mc,
                       cb ? p.heavy_b : p.heavy_a, hc, gwarp, nwarps);
-        local_walk(p, X, p.walk ? kWalkRounds : kTriedRounds, p.walk ? kWalkLight : kTriedLight,
+        local_walk(p, X, p.walk ? kWalkRounds : tried_rounds(n), p.walk ? kWalkLight : kTriedLight,
                    p.walk ? kWalkMed : kTriedMed);
         if (!grid_barrier(c, bar)) return;
         ++level;

@@ -71,6 +71,39 @@ def test_committed_weights_beat_the_heuristic_on_heldout_traces():
     assert report["learned_ms"] <= report["default_ms"]
 
 
+def test_committed_weights_slow_no_recorded_workload_down():
+    # per graph, over the batches that training did not see: the grids too, where the fastest of the
+    # settings is a matter of chance and a wrong one costs a multiple
+    paths = [TRACES, os.path.join(S.DATA_DIR, "scheduler_traces_grid4096.npz")]
+    parts = []
+    for path in paths:
+        with np.load(path) as z:
+            parts.append({k: z[k] for k in z.files})
+    traces = S.merge_traces(parts)
+    with np.load(S.PRETRAINED) as z:
+        pred = S.within_range(S.classes_of(S.reference_forward(
+            z["params"], z["feature_mean"], z["feature_scale"], traces["features"])),
+            traces["features"], z["feature_lo"], z["feature_hi"])
+    hold = S.holdout_mask(traces)
+    for k, name in enumerate(traces["workload_names"]):
+        report = S.evaluate(pred, traces, hold & (traces["workload"] == k))
+        assert report["learned_ms"] <= report["default_ms"], (str(name), report)
+
+
+def test_labels_keep_the_plain_schedule_within_the_margin():
+    settings = np.asarray(S.all_settings(), np.int32)
+    plain = settings.tolist().index(list(S.DEFAULT_CLASSES))
+    times = np.full((3, 96), 2.0)
+    times[0, 5], times[0, plain] = 1.0, 1.05
+    times[1, 7], times[1, plain] = 1.0, 1.2
+    times[2, plain] = 0.5
+    traces = {"settings": settings, "times": times}
+    assert S.labels_of(traces).tolist() == [settings[5].tolist(), settings[7].tolist(),
+                                            list(S.DEFAULT_CLASSES)]
+    assert S.labels_of(traces, 0.1).tolist() == [list(S.DEFAULT_CLASSES), settings[7].tolist(),
+                                                 list(S.DEFAULT_CLASSES)]
+
+
 def test_outside_the_trained_range_the_plain_schedule_runs():
     x = np.zeros((3, 12), np.float32)
     x[1, 5] = 30.0   # a graph far larger than any in training

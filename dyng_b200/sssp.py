@@ -42,11 +42,12 @@ class Options:
 class Schedule:
     """The schedule of one update (what the learned scheduler picks; never changes results)."""
 
-    delta: int = 0
-    grid_blocks: int = 0
-    invalidation: int = 0
-    small_frontier: int = 0
-    heavy_degree: int = 0
+    delta: int = 0           # near-far bucket width (0: from the options)
+    grid_blocks: int = 0     # persistent grid (0: by the graph's vertices and edges)
+    invalidation: int = 0    # 0: by the batch (a short walk, pointer jumping); 1: the subtree walk
+    small_frontier: int = 0  # near frontiers of at most this many light rows (64 x as many below
+    #                          six edges per vertex) stay with their blocks (0: 256, < 0: off)
+    heavy_degree: int = 0    # rows longer than this are split across warps (0: 256)
     record_features: bool = False  # report the learned scheduler's features in the stats
 
     def _to_native(self) -> N.Schedule:
@@ -69,14 +70,14 @@ class Stats:
                   "pj_seeded", "pull_atomics", "pull_appends", "pair_visits", "walk_rows",
                   "walk_slots", "stamps_scanned")
     # Algorithmic bytes per unit of work (4-byte ids / weights, 8-byte packed words and rows):
-    #   pointer-jumping visit 8 (ancestor + flag), jump 12 (ancestor[a], flag[a], write),
+    #   pointer-jumping visit 8 (list entry, or ancestor read and written), jump 4 (ancestor[a]),
     #   invalidated vertex 12 (word set to INF, candidate entry), pull candidate / pushed vertex
     #   20 (list entry, row descriptor, own word), row slot 8 (column + weight), word read 8,
     #   successful atomicMin 8, frontier append 12 (entry + stamp), compared vertex 20 (word, old
     #   distance and parent), seeded vertex 12 (stamp, parent, ancestor written), change pair 16
     #   (list entry, flags, key), walk row 12 (entry, descriptor), walk slot 8 (column, parent),
     #   scanned change stamp 4; attempted atomics and the balance probes are diagnostics (0 bytes).
-    WORK_BYTES = ((8, 12, 12, 20, 8, 8, 20, 8, 8, 8, 12, 20) + (0,) * 10 +
+    WORK_BYTES = ((8, 4, 12, 20, 8, 8, 20, 8, 8, 8, 12, 20) + (0,) * 10 +
                   (12, 8, 12, 16, 12, 8, 4) + (0,) * 3)
     # The work counters of each phase of the kernel (indices into WORK_NAMES), and the phases'
     # device times (indices into PHASES): the per-phase roofline.

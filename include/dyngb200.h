@@ -115,7 +115,7 @@ typedef struct dyngb200_stats {
   int64_t delta;       /* near-far width that ran */
   int64_t max_weight;  /* bound weight of the packing */
   int32_t grid_blocks; /* persistent grid that ran (operators engine: its launches' grid) */
-  int32_t invalidation; /* 0 pointer jumping, 1 subtree walk */
+  int32_t invalidation; /* 0 pointer jumping (a walk that it finished included), 1 subtree walk */
   float apply_ms;      /* device time of the batch applier */
   float sssp_ms;       /* device time of the sssp kernel */
   int64_t rounds;      /* pointer-jumping rounds */
@@ -170,12 +170,15 @@ typedef struct dyngb200_options {
 
 /* The schedule of one update: what the learned scheduler chooses.  A tunable only: every field
  * changes the order of work, never the distances or parents.  Zero fields mean "the fixed
- * heuristic": delta from the options, the occupancy grid, pointer-jumping invalidation. */
+ * heuristic": delta from the options, the grid and the invalidation by the graph's size and the
+ * batch. */
 typedef struct dyngb200_schedule {
   int64_t delta;          /* near-far bucket width (0: heuristic) */
-  int32_t grid_blocks;    /* persistent grid size (0: occupancy x SMs, fewer on small graphs) */
-  int32_t invalidation;   /* 0 heuristic: pointer jumping, or the subtree walk where few tree edges
-                           * of a dense graph changed; 1 subtree walk */
+  int32_t grid_blocks;    /* persistent grid size (0: occupancy x SMs, or where that is less a block
+                           * per 384 vertices or per 4,096 edges) */
+  int32_t invalidation;   /* 0 heuristic: pointer jumping, after a short subtree walk where few tree
+                           * edges of a graph of six or more edges per vertex changed; 1 subtree
+                           * walk */
   int32_t small_frontier; /* near frontiers of at most this many light rows (64 x as many on graphs
                            * of less than six edges per vertex) stay with the blocks that found
                            * them for several rounds (0: 256, < 0: off) */

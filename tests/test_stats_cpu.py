@@ -52,9 +52,10 @@ def test_phase_bytes_add_up_to_the_total():
 def test_bytes_per_unit():
     names = S.Stats.WORK_NAMES
     per_unit = dict(zip(names, S.Stats.WORK_BYTES))
-    # ancestor + flag per visit; list entry, row descriptor and own word per pull candidate and
+    # an entry, or an ancestor read and written, per visit, and the one word that a jump gathers;
+    # list entry, row descriptor and own word per pull candidate and
     # per pushed vertex; column + weight per slot; one packed word per read and per atomicMin
-    assert per_unit["round_visits"] == 8 and per_unit["jumps"] == 12
+    assert per_unit["round_visits"] == 8 and per_unit["jumps"] == 4
     assert per_unit["pull_candidates"] == 20 and per_unit["pushes"] == 20
     assert per_unit["pull_slots"] == 8 and per_unit["push_slots"] == 8
     assert per_unit["push_words"] == 8 and per_unit["atomics"] == 8

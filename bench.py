@@ -441,11 +441,12 @@ def main():
 
     arms = {}
     g_snap, t_snap = g.clone(), tree.clone()
+    # from here on: the arms alone take a few tenths of a second, too few samples of 0.1 s
+    sampler = ClockSampler(local)
+    sampler.start()
     run_arm(env, Arm("generate", schedule=fixed), generate)
     g.copy_from(g_snap)
     tree.copy_from(t_snap)
-    sampler = ClockSampler(local)
-    sampler.start()
     arms["plain"] = run_arm(env, Arm("plain", schedule=fixed), lambda i: recorded[i],
                             nvtx=args.schedule == "plain")
     same = None

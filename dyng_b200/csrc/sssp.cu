@@ -842,9 +842,10 @@ __device__ __forceinline__ int tried_rounds(long long n) {
 
 // Pointer jumping starts from a sequential pass that lays out every vertex's ancestor, except on
 // graphs of at most kPjShort vertices, whose first round reads the stamps and parents itself: a
-// barrier less, two random words per gather instead of one.  Invalidation with 4 rounds, the pass
-// and one hop per round before, now: 41 -> 31 us at 262,144 vertices / 10k changes, 28 -> 16 at
-// 12,345 / 601; at 1,048,576 vertices leaving the pass out measured 60 us, keeping it 56.
+// barrier less, two random words per gather instead of one.  Invalidation with the pass and without,
+// a hundredth of the tree's edges cut: 16,384 vertices 24-26 and 22-25 us, 65,536 26-28 and 24-26,
+// 196,608 35-39 and 32-36, 262,144 41-43 and 39, 393,216 48 and 46-47, 524,288 55-59 and 55-58,
+// 1,048,576 73-75 and 78-80, 2,097,152 118 and 130-134.
 constexpr long long kPjShort = 1LL << 18;
 
 // A block's own levels of the walk: the subtrees below the vertices that it invalidated (a vertex

@@ -225,6 +225,32 @@ def test_the_default_classes_are_the_plain_schedule(D):
     assert np.array_equal(tree.distances, want[0]) and np.array_equal(tree.parents, want[1])
 
 
+@pytest.mark.parametrize("shape,n,size", [("grid", 6400, 40), ("grid", 6400, 900), ("dense", 600, 30),
+                                          ("hub", 5000, 20), ("hub", 5000, 2500), ("chain", 4000, 60)])
+def test_learned_schedules_on_the_branches_that_size_and_batch_choose(D, shape, n, size):
+    # blocks that go on by themselves, short walks, grids by edges: under classes drawn at random
+    from dyng_b200 import scheduler as S
+    rng = np.random.default_rng(n + size)
+    n, s, d, w = random_graph(rng, shape, n)
+    g1, g2 = (D.Graph.from_edges(s, d, w, num_vertices=n) for _ in range(2))
+    t1, t2 = D.sssp.compute(g1, 0), D.sssp.compute(g2, 0)
+    sch = S.Scheduler(seed=6)
+    seen = set()
+    for step in range(10):
+        sch.set_params((rng.normal(size=S.num_params()) * 0.5).astype(np.float32))
+        b = _batch(D, random_batch(rng, n, s, d, size, tree_parents=t1.parents))
+        st1 = D.sssp.update(g1, b, t1)
+        st2 = D.sssp.update(g2, b, t2, scheduler=sch)
+        assert np.array_equal(t1.distances, t2.distances)
+        assert np.array_equal(t1.parents, t2.parents)
+        assert (st1.invalidated, st1.affected) == (st2.invalidated, st2.affected)
+        want = S.schedule_for(st2.schedule_classes, st1.delta, st1.grid_blocks)
+        assert st2.delta == want.delta
+        assert st2.grid_blocks == (want.grid_blocks or st1.grid_blocks)
+        seen.add(tuple(st2.schedule_classes))
+    assert len(seen) >= 2
+
+
 def test_outside_its_trained_range_the_scheduler_keeps_the_plain_schedule(D):
     from dyng_b200 import scheduler as S
     rng = np.random.default_rng(12)

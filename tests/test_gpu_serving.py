@@ -65,10 +65,12 @@ def test_mix_equals_alone(learned, lanes):
     results = {}
 
     def submitter(which):
-        # each thread owns some graphs, so each graph's batches arrive in order
+        # each thread owns some graphs, so each graph's batches arrive in order; all of a thread's
+        # batches are submitted before it waits for the first, so that batches of different graphs
+        # are there together however the threads are scheduled
+        tickets = {i: [server.submit(slots[i], _batch(b)) for b in work[i][1]] for i in which}
         for i in which:
-            tickets = [server.submit(slots[i], _batch(b)) for b in work[i][1]]
-            results[i] = [server.wait(tk) for tk in tickets]
+            results[i] = [server.wait(tk) for tk in tickets[i]]
 
     threads = [threading.Thread(target=submitter, args=([0, 2],)),
                threading.Thread(target=submitter, args=([1, 3],))]

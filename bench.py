@@ -55,7 +55,7 @@ def parse():
                     help="the headline arm; both arms run when scheduler weights exist")
     ap.add_argument("--scheduler-weights", default=os.path.join(ROOT, "dyng_b200", "data",
                                                                 "scheduler_weights.npz"))
-    ap.add_argument("--invalidation", type=int, default=0, help="0 pointer jumping, 1 subtree walk")
+    ap.add_argument("--invalidation", type=int, default=0, help="0 by the batch, 1 subtree walk")
     ap.add_argument("--delta", type=int, default=0)
     ap.add_argument("--grid-blocks", type=int, default=0)
     ap.add_argument("--heavy-degree", type=int, default=0)
